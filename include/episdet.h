@@ -67,12 +67,13 @@ enum { EPISDET_ENGINE_AUTO = 0, EPISDET_ENGINE_TENSOR = 1, EPISDET_ENGINE_SIMT =
 #define EPISDET_FLAG_NO_VALIDATE 0x2u  /* skip the padding / plane-overlap check */
 #define EPISDET_FLAG_TIMING 0x4u       /* time every counting-kernel launch (result.count_kernel_ms) */
 /* Pick the triplet kernel instance for this shape by measurement: the first
- * search of a shape (order, score, log2 of the smaller class) times the plain
- * and the segment-staging instance on the first 8 first SNPs of its own data
- * and keeps the faster; the choice is cached for the process and, when the
- * environment variable EPISDET_TUNE_CACHE names a file, read from and appended
- * to it.  Without the flag the instance follows a fixed rule (staging from
- * classes of 32,768 samples).  Results are the same either way. */
+ * search of a shape (order, score, log2 of the smaller class) times the
+ * instances with wide (112) and narrow (56 third SNPs) tiles on the first 8
+ * first SNPs of its own data and keeps the faster; the choice is cached for
+ * the process and, when the environment variable EPISDET_TUNE_CACHE names a
+ * file, read from and appended to it.  Without the flag the instance follows
+ * a fixed rule (narrow tiles for panels of few SNPs).  Results are the same
+ * either way. */
 #define EPISDET_FLAG_AUTOTUNE 0x8u
 /* Testing aid for failure detection: the tensor engine's scoring warps first
  * wait for a device word that nothing ever sets, so every counting launch
@@ -80,11 +81,10 @@ enum { EPISDET_ENGINE_AUTO = 0, EPISDET_ENGINE_TENSOR = 1, EPISDET_ENGINE_SIMT =
  * memory and returns; the call then fails with EPISDET_ERR_TIMEOUT and the
  * device stays usable for the next call. */
 #define EPISDET_FLAG_INJECT_STALL 0x10u
-/* K2 triplet searches on the tensor engine bound each set's score without
- * table reads and score exactly only the sets that can still enter the top-k
- * list (same results either way).  By default this runs when every CTA scores
- * far more sets than its candidate list holds (about 1.5e9 sets in the
- * search); these flags force it on or off. */
+/* Searches on the tensor engine bound each set's score without table reads
+ * and score exactly only the sets that can still enter the top-k list (same
+ * results either way).  FILTER_OFF scores every set exactly; FILTER_ON, the
+ * default, is the bound (classes past 2^22 samples are scored exactly). */
 #define EPISDET_FLAG_FILTER_ON 0x20u
 #define EPISDET_FLAG_FILTER_OFF 0x40u
 /* episdet_search_perm with order 2 on the tensor engine counts, per label,
@@ -151,8 +151,8 @@ typedef struct episdet_result {
     uint64_t kernel_launches; /* kernels this call launched */
     double count_kernel_ms;   /* EPISDET_FLAG_TIMING: summed device time of the counting launches */
     int64_t count_kernel_launches; /* launches of the counting kernel */
-    double executed_macs;     /* EPISDET_FLAG_TIMING: MACs the tensor engine issued (u8 for pairs and the
-                                 pair table, e2m1 for triplets; 0 for SIMT) */
+    double executed_macs;     /* EPISDET_FLAG_TIMING: e2m1 MACs the tensor engine issued in its counting
+                                 launches (0 for SIMT) */
     int64_t h2d_bytes;        /* host->device bytes this call copied */
     int64_t d2h_bytes;        /* device->host bytes this call copied */
     /* Optional caller-owned outputs of capacity top_capacity (may be NULL). */
@@ -270,8 +270,8 @@ episdet_status episdet_generate_cohort(uint64_t seed, int32_t num_snps, int32_t 
 episdet_status episdet_generate_labels(uint64_t seed, int32_t num_samples, int32_t num_cases, int32_t num_labels,
                                        uint32_t* labels);
 
-/* The cached EPISDET_FLAG_AUTOTUNE choice for a shape: 1 = segment-staging
- * triplet instance, 0 = plain instance, -1 = not tuned yet. */
+/* The cached EPISDET_FLAG_AUTOTUNE choice for a shape: 1 = wide triplet
+ * tiles, 0 = narrow ones, -1 = not tuned yet. */
 int32_t episdet_tuned_stage(int32_t order, int32_t score, int32_t num_cases, int32_t num_controls);
 
 uint64_t episdet_n_choose_k(uint32_t n, uint32_t k);

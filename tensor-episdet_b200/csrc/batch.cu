@@ -227,15 +227,15 @@ extern "C" episdet_status episdet_search_perm(const episdet_cohort* cohort, cons
     const bool on_device = cohort->memory == EPISDET_DEVICE;
     // Label mode: the pair totals of the whole cohort, once, shared read-only
     // by every lane (the computation ends with a synchronise of lane 0's stream).
-    const uint4* tot = nullptr;
-    const size_t tot_bytes = sizeof(uint4) * (size_t)M * (size_t)M;
+    const float4* tot = nullptr;
+    const size_t tot_bytes = sizeof(float4) * (size_t)M * (size_t)M;
     if (o.order == 2 && o.engine != EPISDET_ENGINE_SIMT && !(o.flags & EPISDET_FLAG_PERM_SPLIT) &&
         n <= kTensorMaxClass && tot_bytes <= (size_t)kLabelTotalsMaxBytes) {
         begin_call(w0, o);
         CUDA_TRY(w0->perm_tot.ensure(tot_bytes));
-        st = tensor_pair_totals(w0, d_planes, M, n, (uint4*)w0->perm_tot.p);
+        st = tensor_pair_totals(w0, d_planes, M, n, (float4*)w0->perm_tot.p);
         if (st != EPISDET_OK) return st;
-        tot = (const uint4*)w0->perm_tot.p;
+        tot = (const float4*)w0->perm_tot.p;
     }
     std::atomic<int32_t> next{0};
     std::atomic<bool> stop{false};

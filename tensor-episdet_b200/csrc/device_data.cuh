@@ -12,13 +12,15 @@ struct DevData {
     int n[2];                 // samples per class
     int M;                    // SNPs
     const int* marg[2];       // [3][M] genotype counts (g2 = n - g0 - g1)
-    const uint4* pair4[2];    // [M][M] AND cells (00,01,10,11) of SNP pair (a<b); 3-way only
+    const uint4* pair4[2];    // [M][M] AND cells (00,01,10,11) of SNP pair (a<b); 3-way SIMT engine only
 };
 
-// Search slot lists: one persistent top-K list per CTA, kept in global memory
-// between launches of the same search.
+// Search slot lists: one persistent candidate list per CTA, kept in global
+// memory between launches of the same search.
 struct Slots {
-    Cand* lists;     // [nslots][k]
+    Cand* lists;     // [nslots][ld]; SIMT engine: ld = k, sorted
+    int ld;
+    Cand* thr;       // [nslots] tensor engine: each list's k-th best entry at its last compaction
     int* counts;     // [nslots]
     int nslots;
     int k;

@@ -296,11 +296,12 @@ extern "C" __global__ void __launch_bounds__(kSimtThreads)
 }
 
 // ------------------------------------------------------------ top-K merge
-// Single CTA: merges every slot list into the global best-k, batch by batch
-// through an 8192-entry bitonic sort in shared memory.
+// One CTA merges every slot's list into the global best-k.
 constexpr int kMergeCap = 8192;
 constexpr int kMergeThreads = 1024;
 constexpr int kRadixBits = 11;
+constexpr int kRadixBins = 1 << kRadixBits;
+static_assert(kMergeThreads == kMergeBlockThreads && kMergeSmem == sizeof(Cand) * kMergeCap, "merge launch shape");
 
 // In-place ascending bitonic sort of buf[0, n) (n a power of two <= kMergeCap).
 __device__ void merge_sort_smem(Cand* buf, int n) {
@@ -321,116 +322,192 @@ __device__ void merge_sort_smem(Cand* buf, int n) {
         }
 }
 
+// The k-th smallest of the values that each(f) hands to f over all threads (at
+// least k of them, below 2^bits): a radix select, 11 bits a pass, the bin of
+// the k-th found by a scan over the block.
+template <class Each>
+__device__ uint64_t block_kth(Each each, int k, int bits, int* hist) {
+    __shared__ int s_warp[32];
+    __shared__ int s_bin, s_need;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    uint64_t prefix = 0, mask = 0;
+    int need = k;
+    for (int top = bits; top > 0;) {
+        const int nb = top < kRadixBits ? top : kRadixBits;
+        const int shift = top - nb;
+        for (int i = t; i < kRadixBins; i += kMergeThreads) hist[i] = 0;
+        __syncthreads();
+        each([&](uint64_t v) {
+            if ((v & mask) == prefix) atomicAdd(&hist[(int)(v >> shift) & ((1 << nb) - 1)], 1);
+        });
+        __syncthreads();
+        const int h0 = hist[2 * t], h1 = hist[2 * t + 1];
+        int x = h0 + h1;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) s_warp[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            const int w = s_warp[lane];
+            int z = w;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xFFFFFFFFu, z, o);
+                if (lane >= o) z += y;
+            }
+            s_warp[lane] = z - w;
+        }
+        __syncthreads();
+        const int below = s_warp[warp] + x - h0 - h1;  // values in bins before 2 t
+        if (below < need && need <= below + h0 + h1) {
+            const int second = need > below + h0;
+            s_bin = 2 * t + second;
+            s_need = need - below - (second ? h0 : 0);
+        }
+        __syncthreads();
+        need = s_need;
+        prefix |= (uint64_t)s_bin << shift;
+        mask |= (uint64_t)((1 << nb) - 1) << shift;
+        top = shift;
+        __syncthreads();
+    }
+    return prefix;
+}
+static_assert(kRadixBins == 2 * kMergeThreads, "two bins a thread");
+
+// Calls f(entry index in S.lists) for this thread's share of the listed candidates.
+template <class F>
+__device__ __forceinline__ void each_listed(const Slots& S, F f) {
+    for (int s = threadIdx.x >> 5; s < S.nslots; s += kMergeThreads / 32) {
+        const int n = S.counts[s];
+        for (int e = threadIdx.x & 31; e < n; e += 32) f((size_t)s * S.ld + e);
+    }
+}
+
+// Lowers the search-wide key *S.gkey to the k-th smallest of n keys of distinct
+// sets (seeds != null; 0xFFFFFFFF = none), or of the listed candidates.
+extern "C" __global__ void __launch_bounds__(kMergeThreads)
+    kth_key_kernel(Slots S, const uint32_t* __restrict__ seeds, int n) {
+    __shared__ int hist[kRadixBins];
+    __shared__ int s_total;
+    if (threadIdx.x == 0) s_total = 0;
+    __syncthreads();
+    auto each = [&](auto f) {
+        if (seeds) {
+            for (int i = threadIdx.x; i < n; i += kMergeThreads) {
+                const uint32_t key = __ldg(seeds + i);
+                if (key != 0xFFFFFFFFu) f((uint64_t)key);
+            }
+        } else {
+            const uint32_t lim = *S.gkey;
+            each_listed(S, [&](size_t idx) {
+                const uint32_t key = S.lists[idx].key;
+                if (key <= lim) f((uint64_t)key);
+            });
+        }
+    };
+    int mine = 0;
+    each([&](uint64_t) { ++mine; });
+    mine = __reduce_add_sync(0xFFFFFFFFu, mine);
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&s_total, mine);
+    __syncthreads();
+    if (s_total < S.k) return;
+    const uint32_t key = (uint32_t)block_kth(each, S.k, 32, hist);
+    if (threadIdx.x == 0) atomicMin(S.gkey, key);
+}
+
 // Exact global top-k of the per-CTA candidate lists, by (key, set).
 //
-// Radix selection first: three 11-bit histogram passes over the keys of every
-// listed candidate find T, the k-th smallest key.  The candidates with key <= T
-// contain the top k; they are gathered and sorted alone.  When ties at T
-// exceed the buffer the kernel falls back to merging the lists chunk by chunk.
+// The listed candidates that the search-wide key does not rule out are
+// gathered into shared memory (if they do not fit: those up to the k-th
+// smallest key, and of the ties at that key the smallest sets), cut to the k
+// best keys by another radix select, and sorted.
 extern "C" __global__ void __launch_bounds__(kMergeThreads) merge_topk_kernel(Slots S, Cand* out, int* out_count) {
     extern __shared__ __align__(16) unsigned char smem[];
     Cand* buf = reinterpret_cast<Cand*>(smem);
-    int* hist = reinterpret_cast<int*>(smem);  // aliases buf while selecting
-    __shared__ uint32_t s_prefix, s_mask;
-    __shared__ int s_need, s_total, s_n;
-    const int k = S.k;
-    const long total = (long)S.nslots * k;
-    auto key_at = [&](long idx, uint32_t& key) -> bool {
-        const int s = (int)(idx / k), e = (int)(idx % k);
-        if (e >= S.counts[s]) return false;
-        key = S.lists[idx].key;
-        return true;
+    __shared__ int hist[kRadixBins];
+    __shared__ int s_n;
+    const int k = S.k, lane = threadIdx.x & 31;
+    uint32_t lim = S.gkey ? *S.gkey : 0xFFFFFFFFu;
+    uint64_t lim_set = ~0ull;  // of candidates at key lim
+    auto listed = [&](const Cand& c) { return c.key < lim || (c.key == lim && c.set <= lim_set); };
+    auto gather = [&]() {
+        if (threadIdx.x == 0) s_n = 0;
+        __syncthreads();
+        each_listed(S, [&](size_t idx) {
+            const Cand c = S.lists[idx];
+            if (listed(c)) {
+                const int slot = atomicAdd(&s_n, 1);
+                if (slot < kMergeCap) buf[slot] = c;
+            }
+        });
+        __syncthreads();
+        const int n = s_n;
+        __syncthreads();
+        return n;
     };
-    if (threadIdx.x == 0) {
-        s_prefix = 0;
-        s_mask = 0;
-        s_need = k;
-        s_total = 0;
-    }
-    __syncthreads();
-    // Number of listed candidates.
-    int mine = 0;
-    for (long idx = threadIdx.x; idx < total; idx += kMergeThreads) {
-        uint32_t key;
-        mine += key_at(idx, key) ? 1 : 0;
-    }
-    atomicAdd(&s_total, mine);
-    __syncthreads();
-    uint32_t thr = 0xFFFFFFFFu;  // keep everything when there are at most k candidates
-    if (s_total > k) {
-        for (int pass = 0; pass < 3; ++pass) {
-            const int shift = pass == 0 ? 21 : (pass == 1 ? 10 : 0);
-            const int bits = pass == 2 ? 10 : kRadixBits;
-            const int nb = 1 << bits;
-            for (int i = threadIdx.x; i < nb; i += kMergeThreads) hist[i] = 0;
+    int n = gather();
+    if (n > kMergeCap) {
+        lim = (uint32_t)block_kth(
+            [&](auto f) {
+                const uint32_t l = lim;
+                each_listed(S, [&](size_t idx) {
+                    const uint32_t key = S.lists[idx].key;
+                    if (key <= l) f((uint64_t)key);
+                });
+            },
+            k, 32, hist);
+        n = gather();
+        if (n > kMergeCap) {
+            // Ties at lim: of those, the sets that make up k.
+            int less = 0;
+            each_listed(S, [&](size_t idx) { less += S.lists[idx].key < lim; });
+            if (threadIdx.x == 0) s_n = 0;
             __syncthreads();
-            const uint32_t prefix = s_prefix, mask = s_mask;
-            for (long idx = threadIdx.x; idx < total; idx += kMergeThreads) {
-                uint32_t key;
-                if (key_at(idx, key) && (key & mask) == prefix) atomicAdd(&hist[(key >> shift) & (nb - 1)], 1);
-            }
+            less = __reduce_add_sync(0xFFFFFFFFu, less);
+            if (lane == 0) atomicAdd(&s_n, less);
             __syncthreads();
-            if (threadIdx.x == 0) {
-                int need = s_need, acc = 0, bin = 0;
-                while (acc + hist[bin] < need) acc += hist[bin++];
-                s_need = need - acc;
-                s_prefix = prefix | ((uint32_t)bin << shift);
-                s_mask = mask | ((uint32_t)(nb - 1) << shift);
-            }
+            const int below = s_n;
             __syncthreads();
+            lim_set = block_kth(
+                [&](auto f) {
+                    const uint32_t l = lim;
+                    each_listed(S, [&](size_t idx) {
+                        if (S.lists[idx].key == l) f(S.lists[idx].set);
+                    });
+                },
+                k - below, 64, hist);
+            n = gather();
         }
-        thr = s_prefix;  // the k-th smallest key
-    }
-    // Gather every candidate with key <= thr.
-    if (threadIdx.x == 0) s_n = 0;
-    __syncthreads();
-    for (long idx = threadIdx.x; idx < total; idx += kMergeThreads) {
-        uint32_t key;
-        if (key_at(idx, key) && key <= thr) {
-            const int slot = atomicAdd(&s_n, 1);
-            if (slot < kMergeCap) buf[slot] = S.lists[idx];
+    } else if (n > k) {
+        const uint32_t kth = (uint32_t)block_kth(
+            [&](auto f) {
+                for (int i = threadIdx.x; i < n; i += kMergeThreads) f((uint64_t)buf[i].key);
+            },
+            k, 32, hist);
+        Cand mine[kMergeCap / kMergeThreads];
+#pragma unroll
+        for (int e = 0; e < kMergeCap / kMergeThreads; ++e) {
+            const int i = (int)threadIdx.x + e * kMergeThreads;
+            mine[e] = i < n ? buf[i] : cand_worst();
         }
-    }
-    __syncthreads();
-    const int n = s_n;
-    if (n <= kMergeCap) {
-        int p2 = 1;
-        while (p2 < n) p2 <<= 1;
-        for (int i = n + (int)threadIdx.x; i < p2; i += kMergeThreads) buf[i] = cand_worst();
+        if (threadIdx.x == 0) s_n = 0;
         __syncthreads();
-        merge_sort_smem(buf, p2);
-        const int r = n < k ? n : k;
-        for (int i = threadIdx.x; i < k; i += kMergeThreads) out[i] = i < r ? buf[i] : cand_worst();
-        if (threadIdx.x == 0) *out_count = r;
-        return;
+#pragma unroll
+        for (int e = 0; e < kMergeCap / kMergeThreads; ++e)
+            if ((int)threadIdx.x + e * kMergeThreads < n && mine[e].key <= kth) buf[atomicAdd(&s_n, 1)] = mine[e];
+        __syncthreads();
+        n = s_n;
     }
-    // Ties at thr overflow the buffer: merge the lists chunk by chunk.
-    const int room = kMergeCap - k;
-    __shared__ int s_r;
-    if (threadIdx.x == 0) s_r = 0;
+    int p2 = 1;
+    while (p2 < n) p2 <<= 1;
+    for (int i = n + (int)threadIdx.x; i < p2; i += kMergeThreads) buf[i] = cand_worst();
     __syncthreads();
-    for (long pos = 0; pos < total; pos += room) {
-        int r = s_r;
-        for (int i = threadIdx.x; i < kMergeCap; i += kMergeThreads) {
-            if (i < r) continue;
-            long idx = pos + (i - r);
-            Cand c = cand_worst();
-            if (i - r < room && idx < total) {
-                int s = (int)(idx / k), e = (int)(idx % k);
-                if (e < S.counts[s]) c = S.lists[idx];
-            }
-            buf[i] = c;
-        }
-        __syncthreads();
-        merge_sort_smem(buf, kMergeCap);
-        if (threadIdx.x == 0) {
-            int m = 0;
-            while (m < k && buf[m].key != 0xFFFFFFFFu) ++m;
-            s_r = m;
-        }
-        __syncthreads();
-    }
-    int r = s_r;
+    merge_sort_smem(buf, p2);
+    const int r = n < k ? n : k;
     for (int i = threadIdx.x; i < k; i += kMergeThreads) out[i] = i < r ? buf[i] : cand_worst();
     if (threadIdx.x == 0) *out_count = r;
 }

@@ -227,7 +227,8 @@ static episdet_status search_locked(const episdet_dataset* data, const episdet_o
     slots.lists = (Cand*)(S + kOffSlots);
     slots.counts = (int*)(S + kOffCounts);
     slots.nslots = grid;
-    slots.k = o.top_k;
+    slots.k = slots.ld = o.top_k;
+    slots.thr = nullptr;
     slots.gkey = nullptr;
     CUDA_TRY(cudaMemsetAsync(slots.counts, 0, sizeof(int) * grid, stream));
     search2_simt_kernel<<<grid, kSimtBlockThreads, kSimtSmem2, stream>>>(D, T, (const int2*)(S + kOffTiles), ntiles,

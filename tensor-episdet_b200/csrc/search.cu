@@ -183,11 +183,6 @@ episdet_status build_tables(Workspace* w, int score, int nc, int nn, ScoreTables
         CUDA_TRY(cudaMemcpyAsync(w->t64.p, t64.data(), sizeof(double) * size, cudaMemcpyHostToDevice, w->st));
         CUDA_TRY(cudaStreamSynchronize(w->st));
         w->h2d += (int64_t)size * (sizeof(float) + sizeof(double));
-        w->k2_margin = 0.0f;
-        if (score == EPISDET_SCORE_K2) {
-            episdet_status st = k2_filter_margin(w, nc, nn, (const float*)w->t32.p, &w->k2_margin);
-            if (st != EPISDET_OK) return st;
-        }
         w->tab_score = score;
         w->tab_nc = nc;
         w->tab_nn = nn;
@@ -199,7 +194,6 @@ episdet_status build_tables(Workspace* w, int score, int nc, int nn, ScoreTables
     T->hy32 = w->hy32;
     T->hy64 = w->hy64;
     T->score = score;
-    T->k2_margin = w->k2_margin;
     return EPISDET_OK;
 }
 
@@ -266,15 +260,18 @@ episdet_status stage_dataset(Workspace* w, const episdet_dataset* d, bool valida
 }
 
 episdet_status prepare_slots(Workspace* w, int nslots, int k, Slots* S) {
-    CUDA_TRY(w->slots.ensure(sizeof(Cand) * (size_t)nslots * k));
-    CUDA_TRY(w->counts.ensure(sizeof(int) * ((size_t)nslots + 1)));
-    CUDA_TRY(cudaMemsetAsync(w->counts.p, 0, sizeof(int) * (size_t)nslots, w->st));
-    CUDA_TRY(cudaMemsetAsync((int*)w->counts.p + nslots, 0xFF, sizeof(int), w->st));
+    // Thresholds, search-wide key (both worst: all ones), counts (zero).
+    const size_t ones = sizeof(Cand) * ((size_t)nslots + 1);
+    CUDA_TRY(w->counts.ensure(ones + sizeof(int) * (size_t)nslots));
+    CUDA_TRY(cudaMemsetAsync(w->counts.p, 0xFF, ones, w->st));
+    CUDA_TRY(cudaMemsetAsync((char*)w->counts.p + ones, 0, sizeof(int) * (size_t)nslots, w->st));
     S->lists = (Cand*)w->slots.p;
-    S->counts = (int*)w->counts.p;
+    S->ld = k;
+    S->thr = (Cand*)w->counts.p;
+    S->gkey = (uint32_t*)((Cand*)w->counts.p + nslots);
+    S->counts = (int*)((char*)w->counts.p + ones);
     S->nslots = nslots;
     S->k = k;
-    S->gkey = (uint32_t*)((int*)w->counts.p + nslots);
     return EPISDET_OK;
 }
 
@@ -293,6 +290,7 @@ static episdet_status run_simt(Workspace* w, const DevData& D0, const ScoreTable
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, search3_simt_kernel, kSimtBlockThreads, kSimtSmem3));
     int grid = w->sms * std::max(per_sm, 1);
+    CUDA_TRY(w->slots.ensure(sizeof(Cand) * (size_t)grid * o.top_k));
     episdet_status st = prepare_slots(w, grid, o.top_k, S);
     if (st != EPISDET_OK) return st;
     std::vector<int2> tiles;
@@ -534,15 +532,10 @@ static void tune_store(int key, int choice) {
 }
 
 // Times both triplet instances on the first 8 first SNPs of this search (two
-// rounds, alternating, minimum per instance) and returns the staged one only
-// when it is more than 3 % faster (probes share the GPU with any concurrent
-// work).  With fewer cases than segment 0 needs to be staged (it holds cases
-// only), the plain one is taken without a probe.
+// rounds, alternating, minimum per instance) and returns the wide one unless
+// the narrow one is more than 3 % faster (probes share the GPU with any
+// concurrent work).
 static episdet_status tune_probe(Workspace* w, const episdet_dataset* data, const episdet_options& o, int* choice) {
-    if (data->num_cases < kStageMinSamples) {
-        *choice = 0;
-        return EPISDET_OK;
-    }
     episdet_options po = o;
     po.flags = (o.flags & ~(EPISDET_FLAG_AUTOTUNE | EPISDET_FLAG_PROGRESS)) | EPISDET_FLAG_TIMING;
     po.first_begin = 0;
@@ -558,7 +551,7 @@ static episdet_status tune_probe(Workspace* w, const episdet_dataset* data, cons
             if (st != EPISDET_OK) return st;
             best[c] = std::min(best[c], r.count_kernel_ms);
         }
-    *choice = best[1] < 0.97 * best[0] ? 1 : 0;
+    *choice = best[0] < 0.97 * best[1] ? 0 : 1;
     return EPISDET_OK;
 }
 

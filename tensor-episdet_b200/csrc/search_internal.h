@@ -42,7 +42,10 @@ struct DevBuf {
 // Sets of regrouped operand buffers of the triplet engine: the regrouping of
 // group g + kXSets - 1 (second stream) overlaps the counting launch of group g.
 constexpr int kXSets = 2;
-constexpr int kXGroup = 4;  // first SNPs per triplet launch (tc::kMaxGroup)
+constexpr int kXGroup = 4;  // first SNPs per triplet launch at least
+constexpr int kGroupTiles = 16;                   // tiles per CTA pair that a triplet launch should have
+constexpr size_t kGroupBytes = (size_t)2 << 30;   // regrouped rows a launch may take for them
+constexpr int kNarrowTileSnps = 448;              // panels up to this size use narrow triplet tiles
 
 struct Workspace {
     int device = 0;
@@ -54,15 +57,18 @@ struct Workspace {
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     std::mutex mu;
     DevBuf bits[2], marg[2], pair4[2], t32, t64, slots, counts, tiles, merged, mcount, fp64, flag;
-    DevBuf pairx[2];      // 3-way tensor engine, Y-blocked pair table: pair rows of the current first SNPs
-    DevBuf planes8;       // unpacked 0/1 byte operand rows (tensor engine)
+    DevBuf ptab, ptabx;   // 3-way tensor engine: pair table, and (Y-blocked) the rows of the current first SNPs
+    DevBuf frows;         // packed e2m1 operand rows of the planes (2-way and pair table)
+    DevBuf rtab;          // counts that cells are derived from, per SNP (tensor engine)
+    DevBuf stash;         // drained count segments (tensor engine)
+    DevBuf seeds;         // seed pass: one key per scoring thread (tensor engine)
     DevBuf planes_t[2];   // sample-major transposed planes per class (3-way tensor engine's regrouping)
-    DevBuf xsub[kXSets * kXGroup];  // per-X sample-regrouped operand rows (tensor engine)
+    DevBuf xsub[kXSets];  // sample-regrouped operand rows of one launch's first SNPs (tensor engine)
     DevBuf xinfo;         // per-X segment tables (tensor engine)
     DevBuf tensor_flag;   // device error / progress words of the tensor engine
-    DevBuf cbuf;          // per-CTA candidate buffers of the filtered triplet kernel
+    DevBuf cbuf;          // per-CTA candidate lists (tensor engine)
     DevBuf perm_tot;      // label-free pair totals of a permutation batch's cohort
-    const uint4* label_tot = nullptr;  // set during a label-mode 2-way search (episdet_search_perm)
+    const float4* label_tot = nullptr;  // set during a label-mode 2-way search (episdet_search_perm)
     DevBuf perm_planes, perm_cls[2], perm_idx;  // phenotype-permutation staging
     DevBuf bin_geno, bin_idx, bin_out[2];       // genotype-matrix binarizer staging
     // Per-call accounting.
@@ -74,15 +80,16 @@ struct Workspace {
     double executed_macs = 0.0;
     std::vector<double> launch_ms, launch_macs;  // EPISDET_FLAG_TIMING: per counting launch of the last call
     int tab_score = -1, tab_nc = -1, tab_nn = -1;
-    int stage_override = -1;  // triplet instance: -1 by the class-size rule, 0 plain, 1 staged
-    float inv32 = 0.0f, hy32 = 0.0f, k2_margin = 0.0f;
+    int stage_override = -1;  // triplet tiles: -1 by the panel-size rule, 0 narrow, 1 wide
+    int pairs[16] = {};       // resident CTA pairs of each counting-kernel instance (0: not asked yet)
+    float inv32 = 0.0f, hy32 = 0.0f;
     double inv64 = 0.0, hy64 = 0.0;
 
     void release_all() {
         for (DevBuf& b : xsub) b.release();
-        DevBuf* all[] = {&bits[0], &bits[1], &marg[0], &marg[1], &pair4[0], &pair4[1], &pairx[0], &pairx[1], &t32,
+        DevBuf* all[] = {&bits[0], &bits[1], &marg[0], &marg[1], &pair4[0], &pair4[1], &ptab, &ptabx, &t32,
                          &t64, &slots,
-                         &counts, &tiles, &merged, &mcount, &fp64, &flag, &planes8, &planes_t[0], &planes_t[1],
+                         &counts, &tiles, &merged, &mcount, &fp64, &flag, &frows, &rtab, &stash, &seeds, &planes_t[0], &planes_t[1],
                          &xinfo,
                          &tensor_flag, &cbuf, &perm_tot, &perm_planes, &perm_cls[0], &perm_cls[1], &perm_idx,
                          &bin_geno, &bin_idx, &bin_out[0], &bin_out[1]};
@@ -92,9 +99,6 @@ struct Workspace {
 };
 
 constexpr int kMaxLanes = 4;  // concurrent cohorts of one batched call
-// Samples of count segment 0 from which the staged triplet instance copies it
-// out of TMEM early (below, that instance runs like the plain one).
-constexpr int kStageMinSamples = 8192;
 episdet_status get_workspace(int device, Workspace** out);
 episdet_status get_workspace_lane(int device, int lane, Workspace** out);
 episdet_status build_tables(Workspace* w, int score, int nc, int nn, ScoreTables* T);
@@ -133,13 +137,9 @@ void begin_call(Workspace* w, const episdet_options& o);
 episdet_status search_locked(Workspace* w, const episdet_dataset* data, const episdet_options& o,
                              episdet_result* result);
 
-// Bound of the K2 scoring filter for a sample count (tensor.cu): measures the
-// filter's largest distance to the FP32 table d_t32 on the device.
-episdet_status k2_filter_margin(Workspace* w, int nc, int nn, const float* d_t32, float* margin);
-
 // Label-free AND cells of every pair of one plane set (tensor.cu), for the
 // label-mode 2-way permutation search.
-episdet_status tensor_pair_totals(Workspace* w, const uint32_t* d_planes, int M, int n, uint4* out);
+episdet_status tensor_pair_totals(Workspace* w, const uint32_t* d_planes, int M, int n, float4* out);
 
 // Sets the tensor engine's kernel attributes on the current device.
 episdet_status tensor_init_attributes();

@@ -146,6 +146,20 @@ __device__ __forceinline__ void tmem_regs_ready(uint32_t (&v)[8]) {
                  : "memory");
 }
 
+__device__ __forceinline__ void tmem_regs_ready16(uint32_t (&v)[16]) {
+    asm volatile(""
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                   "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
+                 :
+                 : "memory");
+}
+// One lane of a converged warp (the same one each time).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+
 // Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows of
 // 128 bytes, 8-row groups 1024 bytes apart (SBO), descriptor version 1.
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {

@@ -25,7 +25,7 @@ ENGINE_AUTO, ENGINE_TENSOR, ENGINE_SIMT = 0, 1, 2
 FLAG_PROGRESS, FLAG_NO_VALIDATE, FLAG_TIMING = 0x1, 0x2, 0x4
 FLAG_AUTOTUNE = 0x8  # measure the triplet instance per shape and cache the choice
 FLAG_INJECT_STALL = 0x10  # testing aid: every tensor launch waits on a word nothing sets and times out
-FLAG_FILTER_ON, FLAG_FILTER_OFF = 0x20, 0x40  # force the K2 triplet scoring filter on / off
+FLAG_FILTER_ON, FLAG_FILTER_OFF = 0x20, 0x40  # bound scores before exact scoring (the default) / score every set exactly
 FLAG_PERM_SPLIT = 0x80  # permutation search: a plain two-class search per label instead of label mode
 
 STATUS = {
@@ -396,8 +396,8 @@ def test_fail_allocation(after: int) -> None:
 
 
 def tuned_stage(order: int, score, num_cases: int, num_controls: int) -> int:
-    """The cached FLAG_AUTOTUNE choice for a shape: 1 staged triplet instance,
-    0 plain, -1 not tuned yet."""
+    """The cached FLAG_AUTOTUNE choice for a shape: 1 wide triplet tiles,
+    0 narrow ones, -1 not tuned yet."""
     sc = {"k2": SCORE_K2, "mi": SCORE_MI}[score] if isinstance(score, str) else int(score)
     return int(lib().episdet_tuned_stage(order, sc, num_cases, num_controls))
 

@@ -1,0 +1,62 @@
+"""The counting kernel at the edges of its tiles, against the oracle.
+
+Tiles are 128 A SNPs x 112 (wide) or 56 (narrow) B SNPs; panels of up to 448
+SNPs run narrow triplet tiles, pairs run narrow tiles when wide ones are fewer
+than the CTA pairs.  Counts pass through a buffer of 16-bit values, or 32-bit
+ones for a first SNP with a kept genotype of more than 65,535 samples.  K is
+cut in blocks of 256 samples per segment.  Everything is exact, so the bar is
+equality; FILTER_OFF scores every set exactly, without the score bound.
+"""
+import pytest
+
+from test_parity_gpu import assert_same
+
+pytestmark = pytest.mark.gpu
+
+
+def check(episdet, oracle, order, M, nc, nn, score, k, maf=(0.05, 0.5), seed=0xC0DE, slab=(0, 0), flags=(0,), **planted):
+    cases, controls = episdet.generate(seed + M, M, nc, nn, maf=maf, **planted)
+    o = oracle.search(cases, controls, nc, nn, order=order, score=score, top_k=k, first_begin=slab[0], first_end=slab[1])
+    for f in flags:
+        r = episdet.search(cases, controls, nc, nn, order=order, score=score, top_k=k, engine="tensor",
+                           first_begin=slab[0], first_end=slab[1], flags=f)
+        assert_same(r, o, k)
+        assert r.sets_evaluated == o["sets"]
+
+
+@pytest.mark.parametrize("score", ["k2", "mi"])
+@pytest.mark.parametrize("order,M", [(2, 2), (3, 3), (3, 56), (3, 57), (3, 113), (2, 127), (2, 129), (3, 129), (2, 1130)])
+def test_tile_edges(episdet, oracle, order, M, score):
+    k = 300
+    check(episdet, oracle, order, M, 257, 511, score, k, flags=(0, episdet.FLAG_FILTER_OFF))
+
+
+@pytest.mark.parametrize("score", ["k2", "mi"])
+@pytest.mark.parametrize("M,slab", [(448, (440, 0)), (449, (0, 1)), (449, (126, 129)), (672, (330, 336))])
+def test_triplet_tile_widths_and_list_edges(episdet, oracle, M, slab, score):
+    check(episdet, oracle, 3, M, 1300, 900, score, 1536, slab=slab)
+
+
+@pytest.mark.parametrize("order,M,slab", [(3, 24, (0, 0)), (3, 460, (3, 4)), (2, 40, (0, 0)), (2, 1500, (700, 703))])
+def test_counts_past_16_bits(episdet, oracle, order, M, slab):
+    check(episdet, oracle, order, M, 170000, 150000, "k2", 64, maf=(0.3, 0.36), slab=slab,
+          flags=(0, episdet.FLAG_FILTER_OFF))
+
+
+@pytest.mark.parametrize("score", ["k2", "mi"])
+def test_more_ties_than_the_merge_holds(episdet, oracle, score):
+    """Every SNP the same: all scores equal, the smallest sets win."""
+    import numpy as np
+
+    cases, controls = episdet.generate(9, 1, 300, 260)
+    M, k = 260, 500
+    cases, controls = np.repeat(cases, M, 0), np.repeat(controls, M, 0)
+    o = oracle.search(cases, controls, 300, 260, order=2, score=score, top_k=k)
+    for flags in (0, episdet.FLAG_FILTER_OFF):
+        assert_same(episdet.search(cases, controls, 300, 260, order=2, score=score, top_k=k, engine="tensor",
+                                   flags=flags), o, k)
+
+
+def test_autotune_keeps_the_answer(episdet, oracle):
+    check(episdet, oracle, 3, 120, 2000, 2100, "k2", 200, flags=(episdet.FLAG_AUTOTUNE, 0))
+    assert episdet.tuned_stage(3, "k2", 2000, 2100) in (0, 1)
