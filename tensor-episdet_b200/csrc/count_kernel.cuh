@@ -15,8 +15,8 @@
 //   warp 1       MMA issuer (even CTA of the pair), never waits for scoring;
 //   warps 2-5    drain: tcgen05.ld of a finished segment, counts packed to 16
 //                bits, written to a two-tile ring in global memory (L2);
-//   warps 6-13   scoring: read the tile's counts back, 8 A SNPs x 4 x 2 B
-//                SNPs per warp step, bound every score, score the survivors.
+//   warps 6-13   scoring: read the tile's counts back, one set per lane, bound
+//                every score, score the survivors.
 //
 // Why this split (measured on a B200, SM at its 1965 MHz maximum): the MMA
 // itself takes N / 2 clocks (56 for N = 112, 112 for N = 224) whatever the
@@ -54,6 +54,8 @@ constexpr int kWideZ = 112, kNarrowZ = 56;  // B SNPs of a tile
 // Candidate list of a CTA (global memory): its fill is checked once per tile,
 // so it holds k entries and a whole tile of offers.
 constexpr int kCapG = 16384;
+static_assert((kTileA / 2) * kNarrowZ % kScoreThreads == 0, "every scoring thread has the same number of sets of a tile");
+static_assert((kTileA / 2) * kWideZ / kScoreThreads <= 32, "a thread's sets of a tile are bits of a word");
 static_assert(kMaxTopK + (kTileA / 2) * kWideZ <= kCapG, "candidate list too small for one tile of offers");
 
 // Waits for work (operand copies, MMA commits, drained segments) give up after
@@ -130,14 +132,18 @@ struct CountParams {
 template <int NZ>
 struct Cfg {
     static constexpr int kN = 2 * NZ;               // accumulator columns of a segment
-    static constexpr int kZG = NZ / 4;              // groups of 4 B SNPs (16 bytes of packed counts per row)
+    static constexpr int kSegWords = (kTileA / 2) * NZ;  // sets of a CTA's tile: 8 (narrow) or 16 bytes of counts per segment
     static constexpr int kKbBytes = kABytes + NZ * kKB;  // one K block: 128 A rows, NZ of the pair's 2 NZ B rows
     static constexpr int kStages = NZ == kWideZ ? 6 : 8;
     static constexpr size_t kSmemBars = (size_t)kStages * kKbBytes;
     static constexpr int kNumBars = 2 * kStages + 9;  // full, empty, tfull[2], tempty[2], sfull[2], sempty[2], drain
     static constexpr size_t kSmemMisc = kSmemBars + ((kNumBars * sizeof(uint64_t) + 63) & ~size_t(63));
     static constexpr size_t kSmemGroup = kSmemMisc + 64;
-    static constexpr size_t kSmemTotal = kSmemGroup + (size_t)kMaxGroup * 48 + 1024;
+    // The tile's row of each derived-cell table: [9][NZ] for the B SNPs, [6][64]
+    // for the A SNPs.
+    static constexpr size_t kSmemXz = kSmemGroup + (size_t)kMaxGroup * 48;
+    static constexpr size_t kSmemXy = kSmemXz + (size_t)9 * NZ * 8;
+    static constexpr size_t kSmemTotal = kSmemXy + (size_t)6 * (kTileA / 2) * 8 + 1024;
     static_assert(kSmemTotal <= 232448, "count_kernel shared memory exceeds 227 KB");
     static_assert(kKbBytes % 1024 == 0, "operand tiles must stay 1024-byte aligned");
     static_assert(2 * kN <= 448, "two accumulators and the block scales in 512 TMEM columns");
@@ -275,8 +281,8 @@ __device__ __forceinline__ float bound_value(const Bound& b) {
 }
 
 // ------------------------------------------------------------ the stash
-// A drained segment: narrow, 16-bit counts of 4 B SNPs x 2 planes per 16 bytes,
-// [group of 4 B SNPs][row]; wide, the FP32 counts, [pair of B SNPs][row].
+// A drained segment, [A SNP][B SNP]: narrow, two words of 16-bit counts (A plane
+// 0, 1), each B planes 0 and 1; wide, four FP32 counts in the same order.
 // 16-bit values come and go by adding 2^23 (exact for any count below it).
 __device__ __forceinline__ uint32_t pack16(uint32_t lo, uint32_t hi) {
     const uint32_t a = __float_as_uint(__uint_as_float(lo) + 8388608.0f);
@@ -287,19 +293,12 @@ __device__ __forceinline__ float unpack16(uint32_t w, int hi, float off) {
     return __uint_as_float(__byte_perm(w, 0x4B000000u, hi ? 0x7632 : 0x7610)) - (8388608.0f - off);
 }
 
-// Counts (plane 0, plane 1) of B SNP 2 * zp + z for the A rows of SNP yl in
-// segment s, row j: the exact values, wherever they are kept.
+// The counts [A plane][B plane] of set `idx` = yl * NZ + z in segment s, exact.
 template <int NZ>
-__device__ __forceinline__ float2 stash_counts(const uint4* slot, int wide, int s, int yl, int j, int zp, int z) {
-    using C = Cfg<NZ>;
-    const int row = 2 * yl + j;
-    if (wide) {
-        const uint4* p = slot + ((size_t)(s * C::kZG * 2 + zp) * kCtaRows + row);
-        return __ldcg(reinterpret_cast<const float2*>(p) + z);
-    }
-    const uint4* p = slot + ((size_t)(s * C::kZG + (zp >> 1)) * kCtaRows + row);
-    const uint32_t w = __ldcg(reinterpret_cast<const uint32_t*>(p) + 2 * (zp & 1) + z);
-    return make_float2((float)(w & 0xFFFFu), (float)(w >> 16));
+__device__ __forceinline__ float4 stash_counts(const uint4* slot, int wide, int s, int idx) {
+    if (wide) return __ldcg(reinterpret_cast<const float4*>(slot) + (size_t)s * Cfg<NZ>::kSegWords + idx);
+    const uint2 w = __ldcg(reinterpret_cast<const uint2*>(slot) + (size_t)s * Cfg<NZ>::kSegWords + idx);
+    return make_float4((float)(w.x & 0xFFFFu), (float)(w.x >> 16), (float)(w.y & 0xFFFFu), (float)(w.y >> 16));
 }
 
 // ------------------------------------------------------------ exact score
@@ -314,7 +313,7 @@ struct LutClamped {
 };
 template <int MODE, int SC, int NZ>
 __device__ __noinline__ float exact_score(const CountParams& P, const uint4* slot, int wide, int ga, int gb, int g,
-                                          int yl, int zp, int z, int arow, int bsnp) {
+                                          int idx, int arow, int bsnp) {
     constexpr int NS = MODE == kTriplets ? 3 : 1;  // genotypes of X
     constexpr int NC = MODE == kTriplets ? 27 : 9;
     int tab[2][NC];
@@ -325,27 +324,23 @@ __device__ __noinline__ float exact_score(const CountParams& P, const uint4* slo
                           : nullptr;
     for (int i = 0; i < NS; ++i) {
         int c4[2][2][2];
-        for (int c = 0; c < 2; ++c)
-            for (int j = 0; j < 2; ++j) {
-                float2 v;
-                if (MODE == kPairs && P.tot && c == 1) {
-                    const float4 t = __ldg(P.tot + (size_t)arow * P.M + bsnp);
-                    v = j ? make_float2(t.z, t.w) : make_float2(t.x, t.y);
-                    c4[c][j][0] = (int)v.x - c4[0][j][0];
-                    c4[c][j][1] = (int)v.y - c4[0][j][1];
-                    continue;
-                }
-                if (i < 2) {
-                    v = stash_counts<NZ>(slot, wide, MODE == kTriplets ? 2 * c + i : c, yl, j, zp, z);
-                    c4[c][j][0] = (int)v.x;
-                    c4[c][j][1] = (int)v.y;
-                } else {
-                    c4[c][j][0] = (int)yz[4 * j + c] - sum[c][j][0];
-                    c4[c][j][1] = (int)yz[4 * j + 2 + c] - sum[c][j][1];
-                }
-                sum[c][j][0] += c4[c][j][0];
-                sum[c][j][1] += c4[c][j][1];
+        for (int c = 0; c < 2; ++c) {
+            int v[4];
+            if (i == 2) {
+                for (int e = 0; e < 4; ++e) v[e] = (int)yz[2 * e + c] - sum[c][e >> 1][e & 1];
+            } else if (MODE == kPairs && P.tot && c == 1) {
+                const float4 t = __ldg(P.tot + (size_t)arow * P.M + bsnp);
+                v[0] = (int)t.x - c4[0][0][0], v[1] = (int)t.y - c4[0][0][1];
+                v[2] = (int)t.z - c4[0][1][0], v[3] = (int)t.w - c4[0][1][1];
+            } else {
+                const float4 t = stash_counts<NZ>(slot, wide, MODE == kTriplets ? 2 * c + i : c, idx);
+                v[0] = (int)t.x, v[1] = (int)t.y, v[2] = (int)t.z, v[3] = (int)t.w;
             }
+            for (int e = 0; e < 4; ++e) {
+                c4[c][e >> 1][e & 1] = v[e];
+                sum[c][e >> 1][e & 1] += v[e];
+            }
+        }
         const float2* rt = P.rt + (size_t)(g * 9 + 3 * i) * P.rt_ld;
         for (int c = 0; c < 2; ++c) {
             auto at = [&](int h, int snp) {
@@ -405,6 +400,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     int* s_count = reinterpret_cast<int*>(smem + C::kSmemMisc + 16);
     Cand* s_thr = reinterpret_cast<Cand*>(smem + C::kSmemMisc + 32);
     GroupSm* s_grp = reinterpret_cast<GroupSm*>(smem + C::kSmemGroup);
+    f2* s_xz = reinterpret_cast<f2*>(smem + C::kSmemXz);
+    f2* s_xy = reinterpret_cast<f2*>(smem + C::kSmemXy);
     volatile int* abort = s_abort;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -620,8 +617,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                     break;
                 }
                 ptx::tc_fence_after();
-                uint4* out = slot + (size_t)(s * C::kZG * (wide ? 2 : 1)) * kCtaRows + row;
                 const bool zero = (emask >> s) & 1;
+                const int odd = lane & 1;
+                const size_t o = (size_t)s * C::kSegWords + (size_t)(row >> 1) * NZ;  // set of this lane's A SNP, B SNP 0
 #pragma unroll 2
                 for (int c = 0; c < C::kN; c += 16) {
                     uint32_t v[16];
@@ -633,16 +631,22 @@ __global__ void __launch_bounds__(kThreads, 1)
                         for (int e = 0; e < 16; ++e) v[e] = 0;
                     }
                     if (wide) {
+                        uint2* out = reinterpret_cast<uint2*>(slot) + 2 * (o + c / 2) + odd;
 #pragma unroll
-                        for (int q = 0; q < 4; ++q)
-                            __stcg(out + (size_t)(c / 4 + q) * kCtaRows,
-                                   make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+                        for (int q = 0; q < 8; ++q) __stcg(out + 2 * q, make_uint2(v[2 * q], v[2 * q + 1]));
                     } else {
+                        // The lanes of an A SNP's two planes swap halves: of each
+                        // four B SNPs the even one writes the first two.
+                        uint2* out = reinterpret_cast<uint2*>(slot) + o + c / 2 + 2 * odd;
 #pragma unroll
-                        for (int q = 0; q < 2; ++q)
-                            __stcg(out + (size_t)(c / 8 + q) * kCtaRows,
-                                   make_uint4(pack16(v[8 * q], v[8 * q + 1]), pack16(v[8 * q + 2], v[8 * q + 3]),
-                                              pack16(v[8 * q + 4], v[8 * q + 5]), pack16(v[8 * q + 6], v[8 * q + 7])));
+                        for (int q = 0; q < 2; ++q) {
+                            const uint32_t w0 = pack16(v[8 * q], v[8 * q + 1]), w1 = pack16(v[8 * q + 2], v[8 * q + 3]);
+                            const uint32_t w2 = pack16(v[8 * q + 4], v[8 * q + 5]), w3 = pack16(v[8 * q + 6], v[8 * q + 7]);
+                            const uint32_t r0 = __shfl_xor_sync(0xFFFFFFFFu, odd ? w0 : w2, 1);
+                            const uint32_t r1 = __shfl_xor_sync(0xFFFFFFFFu, odd ? w1 : w3, 1);
+                            __stcg(reinterpret_cast<uint4*>(out + 4 * q),
+                                   odd ? make_uint4(r0, w2, r1, w3) : make_uint4(w0, r0, w1, r1));
+                        }
                     }
                 }
                 ptx::tc_fence_before();
@@ -659,8 +663,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else {
         // ---------------------------------------------------- scoring
         const int etid = threadIdx.x - (64 + 32 * kDrainWarps);
-        const int yl = (warp - 2 - kDrainWarps) * 8 + (lane & 7);  // this thread's A SNP of the CTA's 64
-        const int zq = lane >> 3;
         const BarNamed bar{1, kScoreThreads};
         const int M = P.M;
         LocalTopK<kCapG, kScoreThreads> tk{P.S.lists + (size_t)blockIdx.x * P.S.ld, s_count, s_thr, P.S.k, etid, P.S.gkey};
@@ -676,19 +678,27 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int g = group_of(P, t);
             const int2 tl = P.tiles[P.list_off[g] + t - P.cum[g]];
             const int wide = s_grp[g].wide;
-            const int arow = tl.x * kTileA + rank * (kTileA / 2) + yl;
+            const int arow0 = tl.x * kTileA + rank * (kTileA / 2);
             const int X = MODE == kTriplets ? P.x0 + g : -1;
-            const bool row_ok = arow < M && (MODE != kTriplets || arow > X) &&
-                                (MODE != kPairs || (arow >= P.first_begin && arow < P.first_end));
             const float2* rt = P.rt + (size_t)(g * 9) * P.rt_ld;
             constexpr int NS = MODE == kTriplets ? 3 : 1;
-            f2 xy[NS][2];
+            // This tile's derived-cell rows, on their way to shared memory.
+            constexpr int kXz = 3 * NS * NZ, kXy = 2 * NS * (kTileA / 2);
+            f2 tx[(kXz + kScoreThreads - 1) / kScoreThreads], ty[(kXy + kScoreThreads - 1) / kScoreThreads];
             if (MODE != kStore) {
 #pragma unroll
-                for (int i = 0; i < NS; ++i)
+                for (int e = 0; e * kScoreThreads < kXz; ++e) {
+                    const int i = etid + e * kScoreThreads, h = i / NZ, snp = tl.y * NZ + i % NZ;
+                    tx[e] = i < kXz && snp < M ? __ldg(reinterpret_cast<const f2*>(rt + (size_t)h * P.rt_ld + snp)) : 0;
+                }
 #pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        xy[i][h] = row_ok ? __ldg(reinterpret_cast<const f2*>(rt + (size_t)(3 * i + h) * P.rt_ld + arow)) : 0;
+                for (int e = 0; e * kScoreThreads < kXy; ++e) {
+                    const int i = etid + e * kScoreThreads, h = i / (kTileA / 2);
+                    const int snp = arow0 + i % (kTileA / 2);
+                    ty[e] = i < kXy && snp < M
+                                ? __ldg(reinterpret_cast<const f2*>(rt + (size_t)(h / 2 * 3 + h % 2) * P.rt_ld + snp))
+                                : 0;
+                }
             }
             // The decision to leave must be uniform over the scoring warps
             // (they meet at a named barrier), so it is taken at one.
@@ -698,6 +708,15 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (bar.any(!w)) {
                 ok = false;
                 break;
+            }
+            if (MODE != kStore) {
+#pragma unroll
+                for (int e = 0; e * kScoreThreads < kXz; ++e)
+                    if (etid + e * kScoreThreads < kXz) s_xz[etid + e * kScoreThreads] = tx[e];
+#pragma unroll
+                for (int e = 0; e * kScoreThreads < kXy; ++e)
+                    if (etid + e * kScoreThreads < kXy) s_xy[etid + e * kScoreThreads] = ty[e];
+                bar();
             }
             const uint4* slot = P.stash + (size_t)blockIdx.x * P.stash_cta + (size_t)(local & 1) * P.stash_slot;
             // The smaller of this CTA's and the search-wide k-th best key so far.
@@ -709,87 +728,120 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (key != 0xFFFFFFFFu) cut = __double2float_rd((double)key_score(key, SC == 1) * P.cut_mul + P.cut_add);
             }
             int hi = 0;
-#pragma unroll 1
-            for (int zp = zq; zp < NZ / 2; zp += 4) {
-                const int b0 = tl.y * NZ + 2 * zp;  // the two B SNPs b0, b0 + 1
-                if (!(row_ok && b0 + 1 > arow && b0 < M)) continue;
-                uint2 u[NSEG][2];
+            uint32_t keep = 0;  // this thread's sets to score exactly, bit = step
+            // Set `etid + step * kScoreThreads` of the tile is A SNP yl, B SNP z.
+            struct Item {
+                int yl, z;
+            };
+            auto next = [](Item it) {
+                it.yl += kScoreThreads / NZ;
+                it.z += kScoreThreads % NZ;
+                if (it.z >= NZ) it.z -= NZ, ++it.yl;
+                return it;
+            };
+            auto valid = [&](Item it) {
+                const int arow = arow0 + it.yl, bsnp = tl.y * NZ + it.z;
+                return bsnp > arow && bsnp < M && (MODE != kTriplets || arow > X) &&
+                       (MODE != kPairs || (arow >= P.first_begin && arow < P.first_end));
+            };
+            // What a step reads from L2, fetched two steps ahead: the packed
+            // counts (narrow stash) and the set's pair-table cells, both
+            // contiguous over the lanes.  (With a lane per A SNP the pair-table
+            // reads of a warp touched 32 rows and took a third of the time.)  A
+            // thread without a set to score there reads other valid memory.
+            struct Fetched {
+                uint2 u[NSEG];
+                float4 y0, y1;
+            };
+            auto fetch = [&](Fetched& f, Item it, int step) {
                 if (!wide) {
 #pragma unroll
                     for (int s = 0; s < NSEG; ++s)
-#pragma unroll
-                        for (int j = 0; j < 2; ++j)
-                            u[s][j] = __ldcg(reinterpret_cast<const uint2*>(
-                                                 slot + ((size_t)(s * C::kZG + (zp >> 1)) * kCtaRows + 2 * yl + j)) +
-                                             (zp & 1));
+                        f.u[s] = __ldcg(reinterpret_cast<const uint2*>(slot) + s * C::kSegWords + etid + step * kScoreThreads);
                 }
+                if constexpr (MODE == kTriplets) {
+                    const size_t o = valid(it) ? (size_t)(arow0 + it.yl - P.yv.r0) * (size_t)P.yv.ld +
+                                                     (size_t)(tl.y * NZ + it.z - P.yv.c0)
+                                               : 0;
+                    ptx::ld_stream8(P.yv.p + 8 * o, f.y0, f.y1);
+                }
+            };
+            constexpr int kSteps = C::kSegWords / kScoreThreads;
+            static_assert(kSteps % 2 == 0, "steps are taken in twos");
+            Item it{etid / NZ, etid % NZ};
+            Fetched fa, fb;
+            fetch(fa, it, 0);
+            fetch(fb, next(it), 1);
+#pragma unroll 1
+            for (int step = 0; step < kSteps; step += 2) {
 #pragma unroll
-                for (int z = 0; z < 2; ++z) {
-                    const int bsnp = b0 + z;
-                    if (!(bsnp > arow && bsnp < M)) continue;
+                for (int half = 0; half < 2; ++half, it = next(it)) {
+                    const Fetched f = half ? fb : fa;
+                    if (step + half + 2 < kSteps) fetch(half ? fb : fa, next(next(it)), step + half + 2);
+                    const bool here = valid(it);
+                    if (!__any_sync(0xFFFFFFFFu, here)) continue;
+                    const int yl = it.yl, arow = arow0 + yl, bsnp = tl.y * NZ + it.z;
                     // Counted cells (cases, controls), plus the score's offset.
                     constexpr float off = MODE == kStore ? 0.0f : kCellOff<SC>;
                     f2 c[NSEG / 2][2][2];
                     if (wide) {
 #pragma unroll
-                        for (int i = 0; i < NSEG / 2; ++i)
-#pragma unroll
-                            for (int j = 0; j < 2; ++j) {
-                                const float2 a = stash_counts<NZ>(slot, 1, i, yl, j, zp, z);
-                                const float2 b = stash_counts<NZ>(slot, 1, NSEG / 2 + i, yl, j, zp, z);
-                                c[i][j][0] = pack2(a.x + off, b.x + off);
-                                c[i][j][1] = pack2(a.y + off, b.y + off);
-                            }
+                        for (int i = 0; i < NSEG / 2; ++i) {
+                            const float4 a = stash_counts<NZ>(slot, 1, i, etid + (step + half) * kScoreThreads);
+                            const float4 b = stash_counts<NZ>(slot, 1, NSEG / 2 + i, etid + (step + half) * kScoreThreads);
+                            c[i][0][0] = pack2(a.x + off, b.x + off);
+                            c[i][0][1] = pack2(a.y + off, b.y + off);
+                            c[i][1][0] = pack2(a.z + off, b.z + off);
+                            c[i][1][1] = pack2(a.w + off, b.w + off);
+                        }
                     } else {
 #pragma unroll
-                        for (int i = 0; i < NSEG / 2; ++i)
-#pragma unroll
-                            for (int j = 0; j < 2; ++j) {
-                                const uint32_t a = z ? u[i][j].y : u[i][j].x;
-                                const uint32_t b = z ? u[NSEG / 2 + i][j].y : u[NSEG / 2 + i][j].x;
-                                c[i][j][0] = pack2(unpack16(a, 0, off), unpack16(b, 0, off));
-                                c[i][j][1] = pack2(unpack16(a, 1, off), unpack16(b, 1, off));
-                            }
+                        for (int i = 0; i < NSEG / 2; ++i) {
+                            const uint2 a = f.u[i], b = f.u[NSEG / 2 + i];
+                            c[i][0][0] = pack2(unpack16(a.x, 0, off), unpack16(b.x, 0, off));
+                            c[i][0][1] = pack2(unpack16(a.x, 1, off), unpack16(b.x, 1, off));
+                            c[i][1][0] = pack2(unpack16(a.y, 0, off), unpack16(b.y, 0, off));
+                            c[i][1][1] = pack2(unpack16(a.y, 1, off), unpack16(b.y, 1, off));
+                        }
                     }
                     if constexpr (MODE == kStore) {
-                        float* o = P.out + (size_t)P.out_n * ((size_t)(arow - P.out_r0) * (size_t)P.out_ld +
-                                                              (size_t)(bsnp - P.out_c0));
-                        float v[8];
+                        if (here) {
+                            float* o = P.out + (size_t)P.out_n * ((size_t)(arow - P.out_r0) * (size_t)P.out_ld +
+                                                                  (size_t)(bsnp - P.out_c0));
+                            float v[8];
 #pragma unroll
-                        for (int j = 0; j < 2; ++j)
+                            for (int j = 0; j < 2; ++j)
 #pragma unroll
-                            for (int k = 0; k < 2; ++k) unpack2(c[0][j][k], v[4 * j + 2 * k], v[4 * j + 2 * k + 1]);
-                        if (P.out_n == 8) {
-                            reinterpret_cast<float4*>(o)[0] = make_float4(v[0], v[1], v[2], v[3]);
-                            reinterpret_cast<float4*>(o)[1] = make_float4(v[4], v[5], v[6], v[7]);
-                        } else {
-                            reinterpret_cast<float4*>(o)[0] = make_float4(v[0], v[2], v[4], v[6]);
+                                for (int k = 0; k < 2; ++k) unpack2(c[0][j][k], v[4 * j + 2 * k], v[4 * j + 2 * k + 1]);
+                            if (P.out_n == 8) {
+                                reinterpret_cast<float4*>(o)[0] = make_float4(v[0], v[1], v[2], v[3]);
+                                reinterpret_cast<float4*>(o)[1] = make_float4(v[4], v[5], v[6], v[7]);
+                            } else {
+                                reinterpret_cast<float4*>(o)[0] = make_float4(v[0], v[2], v[4], v[6]);
+                            }
                         }
                         continue;
                     }
                     Bound bd;
-                    auto xz = [&](int i, int h) {
-                        return __ldg(reinterpret_cast<const f2*>(rt + (size_t)(3 * i + h) * P.rt_ld + bsnp));
-                    };
+                    auto xz = [&](int i, int h) { return s_xz[(3 * i + h) * NZ + it.z]; };
+                    auto xy = [&](int i, int h) { return s_xy[(2 * i + h) * (kTileA / 2) + yl]; };
                     if constexpr (MODE == kTriplets) {
-                        const float4* yp = reinterpret_cast<const float4*>(
-                            P.yv.p + 8 * ((size_t)(arow - P.yv.r0) * (size_t)P.yv.ld + (size_t)(bsnp - P.yv.c0)));
-                        const float4 y0 = __ldg(yp), y1 = __ldg(yp + 1);
-                        bound_slice<SC>(bd, c[0], xy[0][0], xy[0][1], xz(0, 0), xz(0, 1), xz(0, 2));
-                        bound_slice<SC>(bd, c[1], xy[1][0], xy[1][1], xz(1, 0), xz(1, 1), xz(1, 2));
+                        bound_slice<SC>(bd, c[0], xy(0, 0), xy(0, 1), xz(0, 0), xz(0, 1), xz(0, 2));
+                        bound_slice<SC>(bd, c[1], xy(1, 0), xy(1, 1), xz(1, 0), xz(1, 1), xz(1, 2));
                         const f2 o3 = pack2(3.0f * off, 3.0f * off);
-                        const f2 yz[2][2] = {{pack2(y0.x, y0.y), pack2(y0.z, y0.w)}, {pack2(y1.x, y1.y), pack2(y1.z, y1.w)}};
+                        const f2 yz[2][2] = {{pack2(f.y0.x, f.y0.y), pack2(f.y0.z, f.y0.w)},
+                                             {pack2(f.y1.x, f.y1.y), pack2(f.y1.z, f.y1.w)}};
                         f2 d[2][2];
 #pragma unroll
                         for (int j = 0; j < 2; ++j)
 #pragma unroll
                             for (int k = 0; k < 2; ++k)
                                 d[j][k] = sub2(sub2(add2(yz[j][k], o3), c[0][j][k]), c[1][j][k]);
-                        bound_slice<SC>(bd, d, xy[2][0], xy[2][1], xz(2, 0), xz(2, 1), xz(2, 2));
+                        bound_slice<SC>(bd, d, xy(2, 0), xy(2, 1), xz(2, 0), xz(2, 1), xz(2, 2));
                     } else {
                         if (P.tot) {
                             // Label mode: controls = all samples - cases.
-                            const float4 t = __ldg(P.tot + (size_t)arow * M + bsnp);
+                            const float4 t = __ldg(P.tot + (here ? (size_t)arow * M + bsnp : 0));
                             const float tv[2][2] = {{t.x, t.y}, {t.z, t.w}};
 #pragma unroll
                             for (int j = 0; j < 2; ++j)
@@ -800,18 +852,28 @@ __global__ void __launch_bounds__(kThreads, 1)
                                     c[0][j][k] = pack2(a, (tv[j][k] + 2.0f * off) - a);
                                 }
                         }
-                        bound_slice<SC>(bd, c[0], xy[0][0], xy[0][1], xz(0, 0), xz(0, 1), xz(0, 2));
+                        bound_slice<SC>(bd, c[0], xy(0, 0), xy(0, 1), xz(0, 0), xz(0, 1), xz(0, 2));
                     }
-                    const float L = bound_value<SC>(bd);
+                    const float L = MODE == kStore ? 0.0f : bound_value<SC>(bd);
+                    if (MODE == kStore || !here) continue;
                     if (P.seeds) {
                         best = fmaxf(best, L);
                         continue;
                     }
-                    if (L < cut) continue;  // provably worse than the k-th candidate
+                    // (Otherwise provably worse than the k-th candidate.)
+                    if (!(L < cut)) keep |= 1u << (step + half);
+                }
+            }
+            // The sets that may enter the list, scored exactly.
+            if constexpr (MODE != kStore) {
+                while (__any_sync(0xFFFFFFFFu, keep != 0)) {
+                    if (keep == 0) continue;
+                    const int e = __ffs((int)keep) - 1;
+                    keep &= keep - 1;
+                    const int idx = etid + e * kScoreThreads, arow = arow0 + idx / NZ, bsnp = tl.y * NZ + idx % NZ;
                     Cand cd;
-                    cd.key = score_key(exact_score<MODE, SC, NZ>(P, slot, wide, s_grp[g].ga, s_grp[g].gb, g, yl, zp, z,
-                                                                 arow, bsnp),
-                                       SC == 1);
+                    cd.key = score_key(
+                        exact_score<MODE, SC, NZ>(P, slot, wide, s_grp[g].ga, s_grp[g].gb, g, idx, arow, bsnp), SC == 1);
                     if (cd.key > lim_key) continue;
                     cd.pad = 0;
                     cd.set = MODE == kTriplets ? set_key3((uint32_t)X, (uint32_t)arow, (uint32_t)bsnp)

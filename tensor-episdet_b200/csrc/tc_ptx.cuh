@@ -74,6 +74,13 @@ __device__ __forceinline__ void prefetch_l2(const void* addr, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(addr), "r"(bytes) : "memory");
 }
 
+// 32 aligned bytes of read-only data that this SM reads once.
+__device__ __forceinline__ void ld_stream8(const float* p, float4& a, float4& b) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p));
+}
+
 // Prefetch of one TMA box into L2 (no shared memory, no completion).
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
     asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y)

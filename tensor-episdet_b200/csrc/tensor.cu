@@ -576,7 +576,7 @@ static episdet_status launch_count(Workspace* w, int inst, const CUtensorMap& ta
 
 // Room for two tiles of drained segments per CTA.
 static episdet_status prepare_stash(Workspace* w, int nz, int nseg, bool wide, CountParams* p) {
-    p->stash_slot = (size_t)nseg * (nz / 4) * kCtaRows * (wide ? 2 : 1);
+    p->stash_slot = (size_t)nseg * nz * (kTileA / 2) / 2 * (wide ? 2 : 1);
     p->stash_cta = 2 * p->stash_slot;
     CUDA_TRY(w->stash.ensure(sizeof(uint4) * p->stash_cta * w->sms));
     p->stash = (uint4*)w->stash.p;
