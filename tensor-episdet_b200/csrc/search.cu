@@ -96,8 +96,12 @@ episdet_status get_workspace_lane(int device, int lane, Workspace** out) {
         Workspace* w = new Workspace();
         w->device = device;
         w->sms = prop.multiProcessorCount;
-        CUDA_TRY(cudaStreamCreateWithFlags(&w->own_st, cudaStreamNonBlocking));
-        CUDA_TRY(cudaStreamCreateWithFlags(&w->aux_st, cudaStreamNonBlocking));
+        // A counting launch goes before the regrouping that becomes ready with
+        // it, which then runs on the SMs that launch frees at its end.
+        int least = 0, greatest = 0;
+        CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        CUDA_TRY(cudaStreamCreateWithPriority(&w->own_st, cudaStreamNonBlocking, greatest));
+        CUDA_TRY(cudaStreamCreateWithPriority(&w->aux_st, cudaStreamNonBlocking, least));
         CUDA_TRY(cudaEventCreateWithFlags(&w->ev_ready, cudaEventDisableTiming));
         for (int i = 0; i < kXSets; ++i) {
             CUDA_TRY(cudaEventCreateWithFlags(&w->ev_cmp[i], cudaEventDisableTiming));

@@ -140,12 +140,11 @@ struct XWork {
     size_t info_bytes;
     int x0;
     int max_n;
-    int* ctr;          // the regrouping's item counter, zeroed here
     __device__ __forceinline__ XInfo* info(int m) const { return reinterpret_cast<XInfo*>(base + m * stride); }
     __device__ __forceinline__ int* idx(int m) const { return reinterpret_cast<int*>(base + m * stride + info_bytes); }
 };
 
-constexpr int kXinfoThreads = 256;
+constexpr int kXinfoThreads = 1024;
 __global__ void __launch_bounds__(kXinfoThreads) xinfo_kernel(DevData D, XWork xw) {
     __shared__ int s_warp[32];
     __shared__ int s_total;
@@ -154,7 +153,6 @@ __global__ void __launch_bounds__(kXinfoThreads) xinfo_kernel(DevData D, XWork x
     XInfo* info = xw.info(blockIdx.y);
     int* idx = xw.idx(blockIdx.y);
     const int max_n = xw.max_n;
-    if (c == 0 && blockIdx.y == 0 && threadIdx.x == 0) *xw.ctr = 0;
     const int M = D.M;
     int tot[3];
 #pragma unroll
@@ -296,22 +294,26 @@ __global__ void __launch_bounds__(kTtThreads) transpose_planes_kernel(DevData D,
 // from tt: a work item is kRgRows rows x 256 packed sample positions (one K
 // block) of one class region of one member.  Each thread copies the 128 bytes
 // of its position's source sample (these rows: one cache line) into shared
-// memory; then each lane transposes one 32 rows x 32 positions block in its
-// own registers (no shuffles) and writes its 32 rows' 16 bytes, the eight
-// lanes of the same rows writing whole 128-byte lines.
+// memory; then each lane transposes one 32 rows x 32 positions block in its own
+// registers (no shuffles) and writes its 32 rows' 16 bytes, the eight lanes of
+// the same rows writing whole 128-byte lines.
+//
+// The bound is DRAM (an eighth of the written bytes read, half a byte per row
+// and kept sample written).  It does not run beside the counting kernel: in a
+// form that fitted there (128 threads, 64 registers) its writes evicted the
+// operands being counted and cost the counting launches of the 4096 x 262144
+// search 1.1 ms for every 0.5 ms saved.
 constexpr int kRgThreads = 256;
 constexpr int kRgRows = 1024;
 constexpr int kRgWords = kRgRows / 32;  // row words per position
-// [position][row word] with 33 words a position and 4 more each 32 positions,
-// so that both the per-position writes and the per-block column reads (lanes
-// of 4 row words x 8 position blocks) are free of bank conflicts.
-__host__ __device__ constexpr int rg_slot(int pos, int q) { return pos * (kRgWords + 1) + 4 * (pos >> 5) + q; }
-constexpr int kRgTBytes = 4 * (rg_slot(kRgThreads - 1, kRgWords - 1) + 1);
-// The allocation also keeps the kernel's CTAs off the SMs of a running
-// counting CTA (172 KB): the regrouping ran beside the counting kernel at the
-// cost of 15 % of the counting rate, more than it saved.
-constexpr int kRgSmem = 64 * 1024;
-static_assert(kRgTBytes <= kRgSmem, "regroup tile");
+constexpr int kRgCtas = 4;              // per SM
+// [position][row word] with 36 words a position and 4 more each 32 positions:
+// 16-byte copies stay aligned, and the per-block column reads (lanes of 4 row
+// words x 8 position blocks) are free of bank conflicts.
+__host__ __device__ constexpr int rg_slot(int pos, int q) { return pos * (kRgWords + 4) + 4 * (pos >> 5) + q; }
+constexpr int kRgSlots = rg_slot(kRgThreads - 1, kRgWords - 1) + 1;
+static_assert(kRgThreads == kF4PerKB, "an item is one K block");
+static_assert(kRgSlots * 4 <= 40 * 1024, "regroup tile");
 
 // 32 x 32 bit transpose of a[0..31] in place: afterwards bit 31 - l of a[k]
 // is what bit 31 - k of a[l] was (the block-swap transpose of H. S. Warren,
@@ -329,103 +331,76 @@ __device__ __forceinline__ void transpose32(uint32_t (&a)[32]) {
     }
 }
 
-// Persistent: a CTA claims work items (member, class K block, row tile) from
-// a launch-wide counter (*ctr, zero at launch), skipping those past a
-// member's region or below its first row, and loads the next item's source
-// samples into registers while it turns the current one into rows.  Claiming
-// (rather than a fixed share per CTA) balances the items over CTAs that start
-// late: the launch begins on the SMs the previous counting launch frees.
-__global__ void __launch_bounds__(kRgThreads, 2)
+// Persistent: CTA i takes items i, i + gridDim.x, ... of the launch's list, in
+// member order, each member's K blocks x its row tiles from row0 on.
+__global__ void __launch_bounds__(kRgThreads, kRgCtas)
     regroup_kernel(DevData D, XWork xw, CmpOut co, const uint32_t* __restrict__ tt0, const uint32_t* __restrict__ tt1,
                    int rwp, int rows_total, int pitch, int nmem) {
-    extern __shared__ __align__(16) uint32_t s_t[];  // rg_slot(position, row word)
-    __shared__ int s_len[kMaxGroup][2][2];           // [member][class][segment]: samples
-    __shared__ int s_claim;
+    __shared__ __align__(16) uint32_t s_t[kRgSlots];  // rg_slot(position, row word)
+    __shared__ int s_len[kMaxGroup][2][2];            // [member][class][segment]: samples
+    __shared__ int s_first[kMaxGroup + 1];            // first item of each member
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    if (t < 4 * nmem) {
-        const int m = t >> 2, c = (t >> 1) & 1, sg = t & 1;
+    for (int i = t; i < 4 * nmem; i += kRgThreads) {
+        const int m = i >> 2, c = (i >> 1) & 1, sg = i & 1;
         s_len[m][c][sg] = xw.info(m)->len[c][sg];
     }
     __syncthreads();
-    const int T0 = (D.W[0] * 32 + kClassPad) / kF4PerKB;
-    const int KT = T0 + (D.W[1] * 32 + kClassPad) / kF4PerKB;
     const int RT = (rows_total + kRgRows - 1) / kRgRows;
-    const int nitems = nmem * KT * RT;
-    // Item i: row tile i % RT, K block (i / RT) % KT of the two class regions,
-    // member i / (RT * KT).  Invalid items are skipped (uniformly).
-    auto decode = [&](int i, int& m, int& c, int& k0, int& rt) -> bool {
-        rt = i % RT;
-        const int kt = (i / RT) % KT;
-        m = i / (RT * KT);
-        c = kt < T0 ? 0 : 1;
-        k0 = (kt - (c ? T0 : 0)) * kF4PerKB;
-        const int pa = (s_len[m][c][0] + kF4PerKB - 1) / kF4PerKB * kF4PerKB;
-        const int pb = (s_len[m][c][1] + kF4PerKB - 1) / kF4PerKB * kF4PerKB;
-        return k0 < pa + pb && (rt + 1) * kRgRows > co.row0[m];
-    };
-    // The next claimed item that is valid (nitems when none is left); called
-    // by every thread, between barriers on s_claim.
-    auto next_valid = [&](int& m, int& c, int& k0, int& rt) {
-        for (;;) {
-            if (t == 0) s_claim = atomicAdd(xw.ctr, 1);
-            __syncthreads();
-            const int i = s_claim;
-            __syncthreads();
-            if (i >= nitems) return nitems;
-            if (decode(i, m, c, k0, rt)) return i;
+    // Positions of a class region: both segments padded to whole K blocks.
+    auto padded = [&](int m, int c, int sg) { return (s_len[m][c][sg] + kF4PerKB - 1) / kF4PerKB * kF4PerKB; };
+    auto blocks = [&](int m, int c) { return (padded(m, c, 0) + padded(m, c, 1)) / kRgThreads; };
+    if (t == 0) {
+        int n = 0;
+        for (int m = 0; m < nmem; ++m) {
+            s_first[m] = n;
+            n += (blocks(m, 0) + blocks(m, 1)) * (RT - co.row0[m] / kRgRows);
         }
-    };
-    // This thread's position of an item: its source sample's 128 bytes of the row tile.
-    auto load = [&](int m, int c, int k0, int rt, uint4 (&v)[kRgWords / 4]) {
-        const int la = s_len[m][c][0], pa = (la + kF4PerKB - 1) / kF4PerKB * kF4PerKB, lb = s_len[m][c][1];
-        const int k = k0 + t;
-        const int* __restrict__ idx = xw.idx(m) + (size_t)c * 2 * xw.max_n;
-        int src = -1;
-        if (k < pa) {
-            if (k < la) src = __ldg(idx + k);
-        } else if (k - pa < lb) {
-            src = __ldg(idx + xw.max_n + (k - pa));
-        }
-        // Row words past the padded row count (the last tile) read as zero.
-        const int nw = min(kRgWords, rwp - rt * kRgWords);
-        const uint4* p =
-            reinterpret_cast<const uint4*>((c ? tt1 : tt0) + (size_t)max(src, 0) * rwp + rt * kRgWords);
-#pragma unroll
-        for (int e = 0; e < kRgWords / 4; ++e)
-            v[e] = (src >= 0 && 4 * e < nw) ? __ldg(p + e) : make_uint4(0, 0, 0, 0);
-    };
+        s_first[nmem] = n;
+    }
+    __syncthreads();
     // This lane's block: row word q (rows 32 q .. 32 q + 31 of the tile) and
     // positions 32 j .. 32 j + 31.
     const int q = 4 * w + (lane >> 3), j = lane & 7;
-    int m, c, k0, rt;
-    int i = next_valid(m, c, k0, rt);
-    uint4 v[kRgWords / 4];
-    if (i < nitems) load(m, c, k0, rt, v);
-    while (i < nitems) {
+    int m = 0;
+    for (int i = blockIdx.x; i < s_first[nmem]; i += gridDim.x) {
+        while (i >= s_first[m + 1]) ++m;
+        const int row0 = co.row0[m], rt0 = row0 / kRgRows, nrt = RT - rt0;
+        const int rt = rt0 + (i - s_first[m]) % nrt, kt = (i - s_first[m]) / nrt;
+        const int b0 = blocks(m, 0), c = kt < b0 ? 0 : 1;
+        const int k0 = (kt - (c ? b0 : 0)) * kRgThreads;
+        {
+            const int la = s_len[m][c][0], pa = padded(m, c, 0), lb = s_len[m][c][1], k = k0 + t;
+            const int* __restrict__ idx = xw.idx(m) + (size_t)c * 2 * xw.max_n;
+            int src = -1;
+            if (k < pa) {
+                if (k < la) src = __ldg(idx + k);
+            } else if (k - pa < lb) {
+                src = __ldg(idx + xw.max_n + (k - pa));
+            }
+            // Row words past the padded row count (the last tile) are zero, as
+            // are positions without a sample.
+            const int nw = src >= 0 ? min(kRgWords, rwp - rt * kRgWords) : 0;
+            const uint32_t* p = (c ? tt1 : tt0) + (size_t)max(src, 0) * rwp + rt * kRgWords;
+            const uint32_t d = ptx::smem_u32(s_t + rg_slot(t, 0));
 #pragma unroll
-        for (int e = 0; e < kRgWords / 4; ++e) {
-            s_t[rg_slot(t, 4 * e)] = v[e].x, s_t[rg_slot(t, 4 * e + 1)] = v[e].y;
-            s_t[rg_slot(t, 4 * e + 2)] = v[e].z, s_t[rg_slot(t, 4 * e + 3)] = v[e].w;
+            for (int e = 0; e < kRgWords / 4; ++e) ptx::cp_async16(d + 16 * e, 4 * e < nw ? p + 4 * e : p, 4 * e < nw);
+            ptx::cp_async_wait_all();
         }
         __syncthreads();
-        const int cm = m, cc = c, ck0 = k0, crt = rt;
-        i = next_valid(m, c, k0, rt);
-        if (i < nitems) load(m, c, k0, rt, v);  // lands while this item is turned into rows
         uint32_t a[32];
         // a[p]: bit 31 - r is row 32 q + r at position 32 j + p.
 #pragma unroll
         for (int p = 0; p < 32; ++p) a[p] = s_t[rg_slot(32 * j + p, q)];
-        transpose32(a);  // a[r]: bit 31 - p is row 32 q + r at position 32 j + p
-        const int row0 = co.row0[cm];
-        uint8_t* __restrict__ out = co.out + (size_t)cm * co.stride +
-                                    ((cc ? D.W[0] * 32 + kClassPad : 0) + ck0) / 2 + 16 * j;
-        const int rbase = crt * kRgRows + 32 * q;
+        __syncthreads();  // s_t may be refilled
+        transpose32(a);   // a[r]: bit 31 - p is row 32 q + r at position 32 j + p
+        uint8_t* __restrict__ out = co.out + (size_t)m * co.stride +
+                                    ((c ? D.W[0] * 32 + kClassPad : 0) + k0) / 2 + 16 * j;
+        const int rbase = rt * kRgRows + 32 * q;
 #pragma unroll
         for (int r = 0; r < 32; ++r) {
             const int row = rbase + r;
             if (row >= row0 && row < rows_total) *reinterpret_cast<uint4*>(out + (size_t)row * pitch) = e2m1_word(a[r]);
         }
-        __syncthreads();  // s_t is refilled next
     }
 }
 
@@ -675,7 +650,6 @@ episdet_status tensor_pair_totals(Workspace* w, const uint32_t* d_planes, int M,
 }
 
 episdet_status tensor_init_attributes() {
-    CUDA_TRY(cudaFuncSetAttribute(regroup_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRgSmem));
     for (int i = 0; i < kInstances; ++i)
         CUDA_TRY(cudaFuncSetAttribute(instance_at(i).kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)instance_at(i).smem));
@@ -937,7 +911,6 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
         xw[b].stride = xstride;
         xw[b].info_bytes = info_bytes;
         xw[b].max_n = max_n;
-        xw[b].ctr = d_err + 2;
         st = make_tmap(&tmx[b][0], w->xsub[b].p, (uint64_t)rows * gmax, (uint64_t)pitch, kCtaRows);
         if (st == EPISDET_OK) st = make_tmap(&tmx[b][1], w->xsub[b].p, (uint64_t)rows * gmax, (uint64_t)pitch, nz);
         if (st != EPISDET_OK) return st;
@@ -949,12 +922,8 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
     int pairs = 0;
     st = resident_pairs(w, inst, &pairs);
     if (st != EPISDET_OK) return st;
-    // Sample-major planes for the regrouping, and its persistent grid (as many
-    // CTAs as fit on the device at once).
+    // Sample-major planes for the regrouping.
     const int rwp = tt_row_words(rows);
-    int rg_per_sm = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rg_per_sm, regroup_kernel, kRgThreads, kRgSmem));
-    const int rg_ctas = std::max(1, rg_per_sm) * grid;
     for (int c = 0; c < 2; ++c) {
         const int warps = (rwp / 8) * (D.W[c] / 8);
         transpose_planes_kernel<<<(warps + kTtThreads / 32 - 1) / (kTtThreads / 32), kTtThreads, 0, w->st>>>(
@@ -1019,7 +988,7 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
             xw[b].x0 = x0;
             xinfo_kernel<<<dim3(2, gn), kXinfoThreads, 0, w->aux_st>>>(D, xw[b]);
             CHECK_LAUNCH();
-            regroup_kernel<<<rg_ctas, kRgThreads, kRgSmem, w->aux_st>>>(
+            regroup_kernel<<<kRgCtas * grid, kRgThreads, 0, w->aux_st>>>(
                 D, xw[b], co[b], (const uint32_t*)w->planes_t[0].p, (const uint32_t*)w->planes_t[1].p, rwp, rows,
                 pitch, gn);
             CHECK_LAUNCH();
