@@ -4,14 +4,11 @@
 // [SNP][genotype 0/1][W] 32-bit words, MSB first, each row zero-padded to a
 // multiple of 1024 bits (src/tensor-episdet.cu:58-148, README.md:48-50).  This
 // builds that layout on the GPU from a dense [SNP][sample] matrix of 0/1/2
-// genotype bytes and a case flag per sample: one thread per output word of a
-// (SNP, class) row packs the 32 samples of that word, taken in sample order
-// within the class through a per-class sample index list.
+// genotype bytes and a case flag per sample.
 #include <cuda_runtime.h>
 
-#include <cstring>
+#include <cstdint>
 #include <mutex>
-#include <vector>
 
 #include "episdet.h"
 #include "host_util.h"
@@ -19,28 +16,89 @@
 
 namespace episdet {
 
-__global__ void __launch_bounds__(256) binarize_kernel(const uint8_t* __restrict__ geno, int M, int n,
-                                                       const int* __restrict__ idx, int n_class, int W,
-                                                       uint32_t* __restrict__ out, int* __restrict__ bad) {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)M * W) return;
-    const int snp = (int)(t / W), w = (int)(t % W);
-    const uint8_t* row = geno + (size_t)snp * n;
-    uint32_t p0 = 0, p1 = 0;
-    int over = 0;
-#pragma unroll 4
-    for (int b = 0; b < 32; ++b) {
-        const int s = w * 32 + b;
-        if (s < n_class) {
-            const uint32_t g = __ldg(row + __ldg(idx + s));
-            p0 |= (uint32_t)(g == 0) << (31 - b);
-            p1 |= (uint32_t)(g == 1) << (31 - b);
+// Sample lists, cases then controls, each in sample order, and *num_cases.
+// One CTA: every thread counts, then lists, one stretch of samples.
+constexpr int kListThreads = 1024;
+__global__ void __launch_bounds__(kListThreads) class_lists_kernel(const uint8_t* __restrict__ is_case, int n,
+                                                                   int* __restrict__ idx, int* __restrict__ num_cases) {
+    __shared__ int s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int per = (n + kListThreads - 1) / kListThreads;
+    const int s0 = min(n, (int)threadIdx.x * per), s1 = min(n, s0 + per);
+    int cnt = 0;
+    for (int i = s0; i < s1; ++i) cnt += __ldg(is_case + i) != 0;
+    int x = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    int below = 0, total = 0;
+    for (int i = 0; i < 32; ++i) {
+        below += i < warp ? s_warp[i] : 0;
+        total += s_warp[i];
+    }
+    int ic = below + x - cnt, in = total + s0 - ic;
+    for (int i = s0; i < s1; ++i) idx[__ldg(is_case + i) != 0 ? ic++ : in++] = i;
+    if (threadIdx.x == 0) *num_cases = total;
+}
+
+// One warp per kBinSnps SNPs x 32 output words of a class: for each word the
+// lanes read the genotypes of its 32 samples (neighbours in the row, so few
+// cache lines) and two ballots make the plane words; lane k keeps word k, so
+// the stores are whole lines.  Reading every genotype byte once is the bound
+// (79 us for 8192 x 50001 at the copy rate); a thread per word, each reading its
+// own 32 samples, took 1.7 ms there.
+constexpr int kBinSnps = 8;
+struct BinClass {
+    const int* idx;  // samples of the class
+    uint32_t* out;   // [M][2][W]
+    int n, W;
+};
+__global__ void __launch_bounds__(256) binarize_kernel(const uint8_t* __restrict__ geno, int M, int n, BinClass a,
+                                                       BinClass b, int* __restrict__ bad) {
+    const int lane = threadIdx.x & 31;
+    const int wa = a.W / 32, wb = b.W / 32;
+    const long unit = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // both classes of an SNP group together
+    const long group = unit / (wa + wb);
+    const int chunk = (int)(unit % (wa + wb));
+    if (group * kBinSnps >= M) return;
+    const bool second = chunk >= wa;
+    const int* __restrict__ idx = second ? b.idx : a.idx;
+    uint32_t* __restrict__ out = second ? b.out : a.out;
+    const int nk = second ? b.n : a.n, W = second ? b.W : a.W;
+    const int w0 = (second ? chunk - wa : chunk) * 32;
+    const int snp0 = (int)group * kBinSnps, ns = min(kBinSnps, M - snp0);
+    const uint8_t* row = geno + (size_t)snp0 * n;
+    uint32_t p0[kBinSnps], p1[kBinSnps];
+#pragma unroll
+    for (int s = 0; s < kBinSnps; ++s) p0[s] = p1[s] = 0;
+    bool over = false;
+#pragma unroll 2
+    for (int k = 0; k < 32; ++k) {
+        const int i = (w0 + k) * 32 + lane;
+        const int at = i < nk ? __ldg(idx + i) : -1;
+#pragma unroll
+        for (int s = 0; s < kBinSnps; ++s) {
+            const uint32_t g = at >= 0 && s < ns ? __ldg(row + (size_t)s * n + at) : 2u;
+            const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, g == 0), m1 = __ballot_sync(0xFFFFFFFFu, g == 1);
             over |= g > 2;
+            if (lane == k) {
+                p0[s] = __brev(m0);
+                p1[s] = __brev(m1);
+            }
         }
     }
-    out[((size_t)snp * 2 + 0) * W + w] = p0;
-    out[((size_t)snp * 2 + 1) * W + w] = p1;
-    if (over) atomicExch(bad, 1);
+#pragma unroll
+    for (int s = 0; s < kBinSnps; ++s)
+        if (s < ns) {
+            uint32_t* o = out + (size_t)(snp0 + s) * 2 * W + w0 + lane;
+            o[0] = p0[s];
+            o[W] = p1[s];
+        }
+    if (__any_sync(0xFFFFFFFFu, over) && lane == 0) atomicExch(bad, 1);
 }
 
 }  // namespace episdet
@@ -64,21 +122,22 @@ extern "C" episdet_status episdet_binarize(const uint8_t* genotypes, int32_t num
     std::lock_guard<std::mutex> lock(w->mu);
     CUDA_TRY(cudaSetDevice(device));
     cudaStream_t s = w->own_st;
-    // Sample index lists, cases first, in sample order.
-    std::vector<uint8_t> flag((size_t)n);
-    if (memory == EPISDET_HOST)
-        memcpy(flag.data(), is_case, (size_t)n);
-    else {
-        CUDA_TRY(cudaMemcpyAsync(flag.data(), is_case, (size_t)n, cudaMemcpyDeviceToHost, s));
-        CUDA_TRY(cudaStreamSynchronize(s));
+    CUDA_TRY(w->bin_idx.ensure(sizeof(int) * (size_t)n + (size_t)n));
+    int* d_idx = (int*)w->bin_idx.p;
+    CUDA_TRY(w->flag.ensure(sizeof(int) * 4));
+    int* d_flag = (int*)w->flag.p;  // [0] a genotype above 2, [1] number of cases
+    CUDA_TRY(cudaMemsetAsync(d_flag, 0, sizeof(int) * 2, s));
+    const uint8_t* d_case = is_case;
+    if (memory == EPISDET_HOST) {
+        uint8_t* f = (uint8_t*)(d_idx + n);
+        CUDA_TRY(cudaMemcpyAsync(f, is_case, (size_t)n, cudaMemcpyHostToDevice, s));
+        d_case = f;
     }
-    std::vector<int> idx((size_t)n);
+    class_lists_kernel<<<1, kListThreads, 0, s>>>(d_case, n, d_idx, d_flag + 1);
+    CHECK_LAUNCH();
     int nc = 0;
-    for (int i = 0; i < n; ++i)
-        if (flag[(size_t)i]) idx[(size_t)nc++] = i;
-    int pos = nc;
-    for (int i = 0; i < n; ++i)
-        if (!flag[(size_t)i]) idx[(size_t)pos++] = i;
+    CUDA_TRY(cudaMemcpyAsync(&nc, d_flag + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
     const int nn = n - nc;
     if (nc < 1 || nn < 1) return set_error(EPISDET_ERR_INVALID_ARGUMENT, "the case flags leave a class empty");
     const int Wc = episdet_class_words(nc), Wn = episdet_class_words(nn);
@@ -95,17 +154,10 @@ extern "C" episdet_status episdet_binarize(const uint8_t* genotypes, int32_t num
             d_out[c] = (uint32_t*)w->bin_out[c].p;
         }
     }
-    CUDA_TRY(w->bin_idx.ensure(sizeof(int) * (size_t)n));
-    CUDA_TRY(w->flag.ensure(sizeof(int) * 4));
-    CUDA_TRY(cudaMemcpyAsync(w->bin_idx.p, idx.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, s));
-    CUDA_TRY(cudaMemsetAsync(w->flag.p, 0, sizeof(int), s));
-    const int ncls[2] = {nc, nn}, Ws[2] = {Wc, Wn};
-    for (int c = 0; c < 2; ++c) {
-        const long threads = (long)M * Ws[c];
-        binarize_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
-            d_geno, M, n, (const int*)w->bin_idx.p + (c ? nc : 0), ncls[c], Ws[c], d_out[c], (int*)w->flag.p);
-        CHECK_LAUNCH();
-    }
+    const BinClass ca{d_idx, d_out[0], nc, Wc}, cb{d_idx + nc, d_out[1], nn, Wn};
+    const long warps = (long)((M + kBinSnps - 1) / kBinSnps) * (Wc / 32 + Wn / 32);
+    binarize_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(d_geno, M, n, ca, cb, d_flag);
+    CHECK_LAUNCH();
     int bad = 0;
     CUDA_TRY(cudaMemcpyAsync(&bad, w->flag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     if (memory == EPISDET_HOST) {

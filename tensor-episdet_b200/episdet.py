@@ -228,8 +228,10 @@ def binarize(genotypes, is_case, device: int = 0):
 
         g = genotypes.contiguous()
         f = (flags != 0).to(torch.uint8).contiguous()
-        cases = torch.zeros((M * 2 * wc,), dtype=torch.int32, device=g.device)
-        controls = torch.zeros((M * 2 * wn,), dtype=torch.int32, device=g.device)
+        cases = torch.empty((M * 2 * wc,), dtype=torch.int32, device=g.device)
+        controls = torch.empty((M * 2 * wn,), dtype=torch.int32, device=g.device)
+        # The library runs on its own stream: what this one still makes must be done.
+        torch.cuda.current_stream(g.device).synchronize()
         _check(lib().episdet_binarize(g.data_ptr(), M, n, f.data_ptr(), cases.data_ptr(), controls.data_ptr(),
                                       DEVICE, device))
         return cases, controls, nc, nn
