@@ -20,6 +20,7 @@
 // the controls' cells are the totals minus the cases'.
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -190,6 +191,25 @@ static episdet_status perm_one(Workspace* w, const uint32_t* d_planes, int M, in
     return st;
 }
 
+// The same in label mode: the classes stay columns of the cohort's planes, only
+// the cases' operand rows are gathered (from the transposed planes), and
+// candidates are re-scored under the class masks.  (Gathering both classes bit
+// by bit took 4 of 10 ms a label at 16384 SNPs x 32768 samples.)
+static episdet_status perm_label(Workspace* w, const LabelCohort& c, const uint32_t* label, const uint32_t* d_label,
+                                 const episdet_options& o, episdet_result* result) {
+    const auto t0 = std::chrono::steady_clock::now();
+    int nc = 0;
+    for (int i = 0; i < c.n / 32; ++i) nc += __builtin_popcount(label[i]);
+    for (int s = c.n / 32 * 32; s < c.n; ++s) nc += (label[s / 32] >> (31 - s % 32)) & 1u;
+    if (nc < 1 || nc >= c.n) return set_error(EPISDET_ERR_INVALID_ARGUMENT, "the label leaves a class empty");
+    reset_result(result);
+    uint64_t launches = 0;
+    DevData D;
+    episdet_status st = tensor_label_rows(w, c, d_label, nc, &D, &launches);
+    if (st == EPISDET_OK) st = search_staged(w, D, o, false, launches, t0, result);
+    return st;
+}
+
 // Label vectors run concurrently on the workspace lanes, like the cohorts of a
 // batch; the cohort's planes are read by every lane from one device copy.
 extern "C" episdet_status episdet_search_perm(const episdet_cohort* cohort, const uint32_t* labels,
@@ -225,18 +245,33 @@ extern "C" episdet_status episdet_search_perm(const episdet_cohort* cohort, cons
         d_planes = (const uint32_t*)w0->perm_planes.p;
     }
     const bool on_device = cohort->memory == EPISDET_DEVICE;
-    // Label mode: the pair totals of the whole cohort, once, shared read-only
-    // by every lane (the computation ends with a synchronise of lane 0's stream).
-    const float4* tot = nullptr;
+    // Label mode: the cohort's transposed planes, genotype counts and pair
+    // totals, once, shared read-only by every lane (the computation ends with a
+    // synchronise of lane 0's stream).
+    LabelCohort lc{d_planes, M, n, W, nullptr, nullptr, nullptr};
     const size_t tot_bytes = sizeof(float4) * (size_t)M * (size_t)M;
-    if (o.order == 2 && o.engine != EPISDET_ENGINE_SIMT && !(o.flags & EPISDET_FLAG_PERM_SPLIT) &&
-        n <= kTensorMaxClass && tot_bytes <= (size_t)kLabelTotalsMaxBytes) {
+    const bool label_mode = o.order == 2 && o.engine != EPISDET_ENGINE_SIMT && !(o.flags & EPISDET_FLAG_PERM_SPLIT) &&
+                            n <= kTensorMaxClass && tot_bytes <= (size_t)kLabelTotalsMaxBytes &&
+                            ((uintptr_t)d_planes & 15) == 0;  // its kernels read 16 bytes at a time
+    const uint32_t* d_labels = labels;
+    std::vector<uint32_t> h_labels;
+    if (label_mode) {
+        // The labels on both sides: the host counts their cases.
+        const size_t words = (size_t)num_labels * W;
+        if (on_device) {
+            h_labels.resize(words);
+            CUDA_TRY(cudaMemcpyAsync(h_labels.data(), labels, sizeof(uint32_t) * words, cudaMemcpyDeviceToHost, w0->own_st));
+        } else {
+            CUDA_TRY(w0->perm_labels.ensure(sizeof(uint32_t) * words));
+            CUDA_TRY(cudaMemcpyAsync(w0->perm_labels.p, labels, sizeof(uint32_t) * words, cudaMemcpyHostToDevice, w0->own_st));
+            d_labels = (const uint32_t*)w0->perm_labels.p;
+        }
+        CUDA_TRY(cudaStreamSynchronize(w0->own_st));
         begin_call(w0, o);
-        CUDA_TRY(w0->perm_tot.ensure(tot_bytes));
-        st = tensor_pair_totals(w0, d_planes, M, n, (float4*)w0->perm_tot.p);
-        if (st != EPISDET_OK) return st;
-        tot = (const float4*)w0->perm_tot.p;
+        st = tensor_label_cohort(w0, &lc, !(o.flags & EPISDET_FLAG_NO_VALIDATE));
+        if (st != EPISDET_OK) return with_prefix(st, "label", 0);
     }
+    const uint32_t* host_labels = on_device ? h_labels.data() : labels;
     std::atomic<int32_t> next{0};
     std::atomic<bool> stop{false};
     std::mutex fail_mu;
@@ -260,10 +295,14 @@ extern "C" episdet_status episdet_search_perm(const episdet_cohort* cohort, cons
             if (p >= num_labels) return;
             clear_error();
             begin_call(w, o);
-            w->label_tot = tot;
-            episdet_status s2 =
-                perm_one(w, d_planes, M, n, W, labels + (size_t)p * W, on_device, p == 0, o, &results[p]);
-            w->label_tot = nullptr;
+            episdet_status s2;
+            if (label_mode) {
+                w->label_tot = lc.tot;
+                s2 = perm_label(w, lc, host_labels + (size_t)p * W, d_labels + (size_t)p * W, o, &results[p]);
+                w->label_tot = nullptr;
+            } else {
+                s2 = perm_one(w, d_planes, M, n, W, labels + (size_t)p * W, on_device, p == 0, o, &results[p]);
+            }
             if (s2 != EPISDET_OK) {
                 std::lock_guard<std::mutex> g(fail_mu);
                 if (fail_p < 0 || p < fail_p) fail_st = s2, fail_p = p, fail_msg = episdet_last_error();

@@ -143,7 +143,8 @@ struct Cfg {
     // for the A SNPs.
     static constexpr size_t kSmemXz = kSmemGroup + (size_t)kMaxGroup * 48;
     static constexpr size_t kSmemXy = kSmemXz + (size_t)9 * NZ * 8;
-    static constexpr size_t kSmemTotal = kSmemXy + (size_t)6 * (kTileA / 2) * 8 + 1024;
+    static constexpr size_t kSmemLevel = kSmemXy + (size_t)6 * (kTileA / 2) * 8;
+    static constexpr size_t kSmemTotal = kSmemLevel + kLevels * sizeof(uint32_t) + 1024;
     static_assert(kSmemTotal <= 232448, "count_kernel shared memory exceeds 227 KB");
     static_assert(kKbBytes % 1024 == 0, "operand tiles must stay 1024-byte aligned");
     static_assert(2 * kN <= 448, "two accumulators and the block scales in 512 TMEM columns");
@@ -362,6 +363,23 @@ __device__ __noinline__ float exact_score(const CountParams& P, const uint4* slo
     return score32_lut<NC, LutClamped, SC>(P.T, LutClamped{P.T.t32, (uint32_t)P.tab_last}, tab[0], tab[1]);
 }
 
+// Counts a scored set of this key at the lowest level it reaches, and lowers
+// the search-wide key to the lowest level that k sets have reached.
+__device__ __noinline__ void reach_level(const Slots& S, const uint32_t* s_level, uint32_t key) {
+    if (key > s_level[0]) return;
+    int j = 0;
+    while (j + 1 < kLevels && key <= s_level[j + 1]) ++j;
+    atomicAdd(&S.level_count[j], 1);
+    int below = 0;
+    for (int i = kLevels - 1; i >= 0; --i) {
+        below += *(volatile int*)&S.level_count[i];
+        if (below >= S.k) {
+            atomicMin(S.gkey, s_level[i]);
+            return;
+        }
+    }
+}
+
 // ------------------------------------------------------------------ kernel
 // MODE kStore (pair table), kPairs (2-way search) or kTriplets; SC the score (0
 // = K2, 1 = MI); NZ the B SNPs of a tile.
@@ -402,6 +420,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     GroupSm* s_grp = reinterpret_cast<GroupSm*>(smem + C::kSmemGroup);
     f2* s_xz = reinterpret_cast<f2*>(smem + C::kSmemXz);
     f2* s_xy = reinterpret_cast<f2*>(smem + C::kSmemXy);
+    uint32_t* s_level = reinterpret_cast<uint32_t*>(smem + C::kSmemLevel);
     volatile int* abort = s_abort;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -670,6 +689,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             *s_count = P.S.counts[blockIdx.x];
             *s_thr = P.S.thr[blockIdx.x];
         }
+        if (MODE != kStore && etid < kLevels) s_level[etid] = P.seeds ? 0 : P.S.level[etid];
         bar();
         float best = -INFINITY;  // seed pass: this thread's largest bound
         bool ok = true;
@@ -765,6 +785,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                                                : 0;
                     ptx::ld_stream8(P.yv.p + 8 * o, f.y0, f.y1);
                 }
+                if (MODE == kPairs && P.tot)
+                    f.y0 = __ldg(P.tot + (valid(it) ? (size_t)(arow0 + it.yl) * M + tl.y * NZ + it.z : 0));
             };
             constexpr int kSteps = C::kSegWords / kScoreThreads;
             static_assert(kSteps % 2 == 0, "steps are taken in twos");
@@ -841,8 +863,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     } else {
                         if (P.tot) {
                             // Label mode: controls = all samples - cases.
-                            const float4 t = __ldg(P.tot + (here ? (size_t)arow * M + bsnp : 0));
-                            const float tv[2][2] = {{t.x, t.y}, {t.z, t.w}};
+                            const float tv[2][2] = {{f.y0.x, f.y0.y}, {f.y0.z, f.y0.w}};
 #pragma unroll
                             for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -875,6 +896,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     cd.key = score_key(
                         exact_score<MODE, SC, NZ>(P, slot, wide, s_grp[g].ga, s_grp[g].gb, g, idx, arow, bsnp), SC == 1);
                     if (cd.key > lim_key) continue;
+                    reach_level(P.S, s_level, cd.key);
                     cd.pad = 0;
                     cd.set = MODE == kTriplets ? set_key3((uint32_t)X, (uint32_t)arow, (uint32_t)bsnp)
                                                : set_key2((uint32_t)arow, (uint32_t)bsnp);

@@ -12,6 +12,9 @@ struct DevData {
     int n[2];                 // samples per class
     int M;                    // SNPs
     const int* marg[2];       // [3][M] genotype counts (g2 = n - g0 - g1)
+    // Label mode: both classes are columns of one plane set (bits[0] = bits[1],
+    // W[0] = W[1]), class c the samples of mask[c] [W]; null otherwise.
+    const uint32_t* mask[2];
     const uint4* pair4[2];    // [M][M] AND cells (00,01,10,11) of SNP pair (a<b); 3-way SIMT engine only
 };
 
@@ -28,7 +31,14 @@ struct Slots {
     // until one held k candidates): a set whose key is larger has k better
     // sets and cannot be in the search's top k.
     uint32_t* gkey;
+    // Tensor engine: descending keys level[0 .. kLevels) below the first
+    // threshold (0 = none) and, from level_count, how many scored sets had a
+    // key in (level[j + 1], level[j]]: once k sets are at or below level[j],
+    // that is the search-wide key.
+    uint32_t* level;
+    int* level_count;
 };
+constexpr int kLevels = 16;
 
 __device__ __forceinline__ void load_marg3(const int* m, int M, int snp, int out[3]) {
     out[0] = __ldg(m + snp);

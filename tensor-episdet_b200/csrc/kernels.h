@@ -22,7 +22,7 @@ extern "C" __global__ void search2_simt_kernel(DevData D, ScoreTables T, const i
                                                uint4* pair_out0, uint4* pair_out1);
 extern "C" __global__ void search3_simt_kernel(DevData D, ScoreTables T, int xsnp, const int2* tiles, int ntiles,
                                                Slots S);
-extern "C" __global__ void kth_key_kernel(Slots S, const uint32_t* seeds, int n);
+extern "C" __global__ void seed_levels_kernel(Slots S, const uint32_t* seeds, int n);
 extern "C" __global__ void merge_topk_kernel(Slots S, Cand* out, int* out_count);
 extern "C" __global__ void rescore_kernel(DevData D, ScoreTables T, int order, const Cand* cands, const int* count,
                                           double* fp64_out, int* cells_out);

@@ -387,36 +387,51 @@ __device__ __forceinline__ void each_listed(const Slots& S, F f) {
     }
 }
 
-// Lowers the search-wide key *S.gkey to the k-th smallest of n keys of distinct
-// sets (seeds != null; 0xFFFFFFFF = none), or of the listed candidates.
+// The first search-wide key from the keys of n distinct sets (0xFFFFFFFF = none):
+// the k-th smallest, and below it the (k / 2)-th, (k / 4)-th, ... as the levels
+// that the counting kernel tightens it to.  Nothing if there are fewer than k.
 extern "C" __global__ void __launch_bounds__(kMergeThreads)
-    kth_key_kernel(Slots S, const uint32_t* __restrict__ seeds, int n) {
+    seed_levels_kernel(Slots S, const uint32_t* __restrict__ seeds, int n) {
     __shared__ int hist[kRadixBins];
-    __shared__ int s_total;
-    if (threadIdx.x == 0) s_total = 0;
-    __syncthreads();
+    __shared__ uint32_t s_key[kRadixBins];
+    __shared__ int s_n;
+    static_assert(kMaxTopK <= kRadixBins, "the seeds at or below the first level fit");
+    const int t = threadIdx.x;
     auto each = [&](auto f) {
-        if (seeds) {
-            for (int i = threadIdx.x; i < n; i += kMergeThreads) {
-                const uint32_t key = __ldg(seeds + i);
-                if (key != 0xFFFFFFFFu) f((uint64_t)key);
-            }
-        } else {
-            const uint32_t lim = *S.gkey;
-            each_listed(S, [&](size_t idx) {
-                const uint32_t key = S.lists[idx].key;
-                if (key <= lim) f((uint64_t)key);
-            });
+        for (int i = t; i < n; i += kMergeThreads) {
+            const uint32_t key = __ldg(seeds + i);
+            if (key != 0xFFFFFFFFu) f((uint64_t)key);
         }
     };
+    if (t == 0) s_n = 0;
+    __syncthreads();
     int mine = 0;
     each([&](uint64_t) { ++mine; });
     mine = __reduce_add_sync(0xFFFFFFFFu, mine);
-    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&s_total, mine);
+    if ((t & 31) == 0 && mine) atomicAdd(&s_n, mine);
     __syncthreads();
-    if (s_total < S.k) return;
-    const uint32_t key = (uint32_t)block_kth(each, S.k, 32, hist);
-    if (threadIdx.x == 0) atomicMin(S.gkey, key);
+    if (s_n < S.k) return;
+    const uint32_t kth = (uint32_t)block_kth(each, S.k, 32, hist);
+    // The smaller ones, sorted (ties at the k-th fill up the rest).
+    for (int i = t; i < kRadixBins; i += kMergeThreads) s_key[i] = kth;
+    if (t == 0) s_n = 0;
+    __syncthreads();
+    each([&](uint64_t v) {
+        if (v < kth) s_key[atomicAdd(&s_n, 1)] = (uint32_t)v;
+    });
+    __syncthreads();
+    for (int kk = 2; kk <= kRadixBins; kk <<= 1)
+        for (int j = kk >> 1; j > 0; j >>= 1) {
+            const int i = ((t & ~(j - 1)) << 1) | (t & (j - 1));  // 1024 pairs of 2048
+            const uint32_t x = s_key[i], y = s_key[i + j];
+            if (((i & kk) == 0) == (x > y)) {
+                s_key[i] = y;
+                s_key[i + j] = x;
+            }
+            __syncthreads();
+        }
+    if (t < kLevels && (S.k >> t) > 0) S.level[t] = s_key[(S.k >> t) - 1];
+    if (t == 0) atomicMin(S.gkey, kth);
 }
 
 // Exact global top-k of the per-CTA candidate lists, by (key, set).
@@ -554,10 +569,12 @@ extern "C" __global__ void __launch_bounds__(256)
         const uint32_t* X1 = X0 + W;
         const uint32_t* Y0 = D.bits[c] + ((size_t)ys * 2 + 0) * W;
         const uint32_t* Y1 = Y0 + W;
+        const uint32_t* mask = D.mask[c];
         if (order == 2) {
             uint32_t a[4] = {0, 0, 0, 0};
             for (int w = lane; w < W; w += 32) {
-                uint32_t x0 = X0[w], x1 = X1[w], y0 = Y0[w], y1 = Y1[w];
+                const uint32_t m = mask ? mask[w] : ~0u;
+                uint32_t x0 = X0[w] & m, x1 = X1[w] & m, y0 = Y0[w], y1 = Y1[w];
                 a[0] += __popc(x0 & y0);
                 a[1] += __popc(x0 & y1);
                 a[2] += __popc(x1 & y0);
@@ -578,7 +595,8 @@ extern "C" __global__ void __launch_bounds__(256)
             uint32_t t8[8] = {0, 0, 0, 0, 0, 0, 0, 0}, pxy[4] = {0, 0, 0, 0}, pxz[4] = {0, 0, 0, 0},
                      pyz[4] = {0, 0, 0, 0};
             for (int w = lane; w < W; w += 32) {
-                uint32_t x[2] = {X0[w], X1[w]}, y[2] = {Y0[w], Y1[w]}, z[2] = {Z0[w], Z1[w]};
+                const uint32_t m = mask ? mask[w] : ~0u;
+                uint32_t x[2] = {X0[w] & m, X1[w] & m}, y[2] = {Y0[w] & m, Y1[w] & m}, z[2] = {Z0[w], Z1[w]};
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
 #pragma unroll

@@ -230,6 +230,8 @@ static episdet_status search_locked(const episdet_dataset* data, const episdet_o
     slots.k = slots.ld = o.top_k;
     slots.thr = nullptr;
     slots.gkey = nullptr;
+    slots.level = nullptr;
+    slots.level_count = nullptr;
     CUDA_TRY(cudaMemsetAsync(slots.counts, 0, sizeof(int) * grid, stream));
     search2_simt_kernel<<<grid, kSimtBlockThreads, kSimtSmem2, stream>>>(D, T, (const int2*)(S + kOffTiles), ntiles,
                                                                           fb, fe, slots, 0, nullptr, nullptr);

@@ -241,6 +241,7 @@ episdet_status stage_dataset(Workspace* w, const episdet_dataset* d, bool valida
         CUDA_TRY(w->marg[c].ensure(sizeof(int) * 3 * (size_t)d->num_snps));
         D->marg[c] = (const int*)w->marg[c].p;
         D->pair4[c] = nullptr;
+        D->mask[c] = nullptr;
     }
     CUDA_TRY(w->flag.ensure(sizeof(int) * 4));
     CUDA_TRY(cudaMemsetAsync(w->flag.p, 0, sizeof(int) * 4, w->st));
@@ -265,15 +266,18 @@ episdet_status stage_dataset(Workspace* w, const episdet_dataset* d, bool valida
 
 episdet_status prepare_slots(Workspace* w, int nslots, int k, Slots* S) {
     // Thresholds, search-wide key (both worst: all ones), counts (zero).
-    const size_t ones = sizeof(Cand) * ((size_t)nslots + 1);
-    CUDA_TRY(w->counts.ensure(ones + sizeof(int) * (size_t)nslots));
+    // Then the threshold levels and their counts (none: zero).
+    const size_t ones = sizeof(Cand) * ((size_t)nslots + 1), zeros = sizeof(int) * ((size_t)nslots + 2 * kLevels);
+    CUDA_TRY(w->counts.ensure(ones + zeros));
     CUDA_TRY(cudaMemsetAsync(w->counts.p, 0xFF, ones, w->st));
-    CUDA_TRY(cudaMemsetAsync((char*)w->counts.p + ones, 0, sizeof(int) * (size_t)nslots, w->st));
+    CUDA_TRY(cudaMemsetAsync((char*)w->counts.p + ones, 0, zeros, w->st));
     S->lists = (Cand*)w->slots.p;
     S->ld = k;
     S->thr = (Cand*)w->counts.p;
     S->gkey = (uint32_t*)((Cand*)w->counts.p + nslots);
     S->counts = (int*)((char*)w->counts.p + ones);
+    S->level = (uint32_t*)(S->counts + nslots);
+    S->level_count = S->counts + nslots + kLevels;
     S->nslots = nslots;
     S->k = k;
     return EPISDET_OK;
@@ -559,6 +563,19 @@ static episdet_status tune_probe(Workspace* w, const episdet_dataset* data, cons
     return EPISDET_OK;
 }
 
+// Clears a result but for the caller's output arrays.
+void reset_result(episdet_result* result) {
+    uint32_t* keep_snps = result->top_snps;
+    float* keep32 = result->top_fp32;
+    double* keep64 = result->top_fp64;
+    int32_t keepcap = result->top_capacity;
+    memset(result, 0, sizeof(*result));
+    result->top_snps = keep_snps;
+    result->top_fp32 = keep32;
+    result->top_fp64 = keep64;
+    result->top_capacity = keepcap;
+}
+
 episdet_status search_locked(Workspace* w, const episdet_dataset* data, const episdet_options& o,
                              episdet_result* result) {
     auto t0 = std::chrono::steady_clock::now();
@@ -582,22 +599,20 @@ episdet_status search_locked(Workspace* w, const episdet_dataset* data, const ep
         w->stage_override = choice;
     }
     begin_call(w, o);
-    uint32_t* keep_snps = result->top_snps;
-    float* keep32 = result->top_fp32;
-    double* keep64 = result->top_fp64;
-    int32_t keepcap = result->top_capacity;
-    memset(result, 0, sizeof(*result));
-    result->top_snps = keep_snps;
-    result->top_fp32 = keep32;
-    result->top_fp64 = keep64;
-    result->top_capacity = keepcap;
-
+    reset_result(result);
     uint64_t launches = 0;
     DevData D;
     episdet_status st = stage_dataset(w, data, !(o.flags & EPISDET_FLAG_NO_VALIDATE), &D, &launches);
     if (st != EPISDET_OK) return st;
+    return search_staged(w, D, o, simt, launches, t0, result);
+}
+
+// The rest of one search, its planes on the device and its marginals computed
+// (or on their way on w->st).
+episdet_status search_staged(Workspace* w, DevData& D, const episdet_options& o, bool simt, uint64_t launches,
+                             std::chrono::steady_clock::time_point t0, episdet_result* result) {
     ScoreTables T;
-    st = build_tables(w, o.score, data->num_cases, data->num_controls, &T);
+    episdet_status st = build_tables(w, o.score, D.n[0], D.n[1], &T);
     if (st != EPISDET_OK) return st;
     const int fb = o.first_begin, fe = o.first_end;
     CUDA_TRY(cudaEventRecord(w->e0, w->st));
@@ -613,8 +628,8 @@ episdet_status search_locked(Workspace* w, const episdet_dataset* data, const ep
     float ms = 0.0f;
     CUDA_TRY(cudaEventElapsedTime(&ms, w->e0, w->e1));
     result->device_ms = ms;
-    result->sets_evaluated = sets_in_slab(o.order, data->num_snps, fb, fe);
-    result->rounds = reference_rounds(o.order, data->num_snps);
+    result->sets_evaluated = sets_in_slab(o.order, D.M, fb, fe);
+    result->rounds = reference_rounds(o.order, D.M);
     result->kernel_launches = launches;
     result->count_kernel_launches = w->count_launches;
     result->executed_macs = w->executed_macs;

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <chrono>
 #include <cmath>
 #include <cstddef>
 #include <cstdint>
@@ -68,6 +69,7 @@ struct Workspace {
     DevBuf tensor_flag;   // device error / progress words of the tensor engine
     DevBuf cbuf;          // per-CTA candidate lists (tensor engine)
     DevBuf perm_tot;      // label-free pair totals of a permutation batch's cohort
+    DevBuf perm_tt, perm_marg, perm_labels, perm_mask;  // label mode: transposed planes, genotype counts, labels, class masks
     const float4* label_tot = nullptr;  // set during a label-mode 2-way search (episdet_search_perm)
     DevBuf perm_planes, perm_cls[2], perm_idx;  // phenotype-permutation staging
     DevBuf bin_geno, bin_idx, bin_out[2];       // genotype-matrix binarizer staging
@@ -91,7 +93,7 @@ struct Workspace {
                          &t64, &slots,
                          &counts, &tiles, &merged, &mcount, &fp64, &flag, &frows, &rtab, &stash, &seeds, &planes_t[0], &planes_t[1],
                          &xinfo,
-                         &tensor_flag, &cbuf, &perm_tot, &perm_planes, &perm_cls[0], &perm_cls[1], &perm_idx,
+                         &tensor_flag, &cbuf, &perm_tot, &perm_tt, &perm_marg, &perm_labels, &perm_mask, &perm_planes, &perm_cls[0], &perm_cls[1], &perm_idx,
                          &bin_geno, &bin_idx, &bin_out[0], &bin_out[1]};
         for (DevBuf* b : all) b->release();
         tab_score = tab_nc = tab_nn = -1;
@@ -136,6 +138,28 @@ void begin_call(Workspace* w, const episdet_options& o);
 // One search; the caller holds w->mu and has validated the options.
 episdet_status search_locked(Workspace* w, const episdet_dataset* data, const episdet_options& o,
                              episdet_result* result);
+
+void reset_result(episdet_result* result);
+episdet_status search_staged(Workspace* w, DevData& D, const episdet_options& o, bool simt, uint64_t launches,
+                             std::chrono::steady_clock::time_point t0, episdet_result* result);
+
+// What every label of a label-mode permutation batch shares: the cohort's
+// planes, their sample-major transpose, its genotype counts [3][M] and its pair
+// totals, all in lane 0's workspace.
+struct LabelCohort {
+    const uint32_t* planes;
+    int M, n, W;
+    const uint32_t* tt;
+    const int* marg;
+    const float4* tot;
+};
+// Fills tt, marg and tot on lane 0 (tensor.cu); EPISDET_ERR_INVALID_INPUT if
+// `validate` and the genotype planes of a sample overlap.
+episdet_status tensor_label_cohort(Workspace* w, LabelCohort* c, bool validate);
+// Class masks, marginals and case operand rows of one label (device words) of
+// nc cases, on w->st; D describes the two classes afterwards (tensor.cu).
+episdet_status tensor_label_rows(Workspace* w, const LabelCohort& c, const uint32_t* d_label, int nc, DevData* D,
+                                 uint64_t* launches);
 
 // Label-free AND cells of every pair of one plane set (tensor.cu), for the
 // label-mode 2-way permutation search.

@@ -210,6 +210,94 @@ __global__ void __launch_bounds__(kXinfoThreads) xinfo_kernel(DevData D, XWork x
     }
 }
 
+// Genotype counts of a whole cohort, [3][M], over its n samples: one warp per
+// SNP.  *bad is set when a sample has both genotype planes.
+__global__ void __launch_bounds__(256) cohort_marginals_kernel(const uint32_t* __restrict__ planes, int M, int n, int W,
+                                                               int* __restrict__ marg, int* __restrict__ bad) {
+    const int snp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (snp >= M) return;
+    const uint32_t* p0 = planes + (size_t)snp * 2 * W;
+    const uint32_t* p1 = p0 + W;
+    int c0 = 0, c1 = 0;
+    uint32_t over = 0;
+    for (int w = lane; w < W; w += 32) {
+        const int lo = w * 32;
+        const uint32_t valid = (lo + 32 <= n) ? 0xFFFFFFFFu : (lo >= n ? 0u : (0xFFFFFFFFu << (32 - (n - lo))));
+        const uint32_t a = __ldg(p0 + w) & valid, b = __ldg(p1 + w) & valid;
+        c0 += __popc(a);
+        c1 += __popc(b);
+        over |= a & b;
+    }
+    c0 = __reduce_add_sync(0xFFFFFFFFu, c0);
+    c1 = __reduce_add_sync(0xFFFFFFFFu, c1);
+    if (over) atomicOr(bad, 1);
+    if (lane == 0) {
+        marg[snp] = c0;
+        marg[M + snp] = c1;
+        marg[2 * M + snp] = n - c0 - c1;
+    }
+}
+
+// One label: the ascending case samples (as member 0's first segment of class
+// 0, the form the regrouping reads) and the two classes' masks.
+__global__ void __launch_bounds__(kXinfoThreads) label_lists_kernel(const uint32_t* __restrict__ label, int n, int W,
+                                                                    XWork xw, uint32_t* __restrict__ mask) {
+    __shared__ int s_warp[32];
+    __shared__ int s_total;
+    const int per = (W + kXinfoThreads - 1) / kXinfoThreads;
+    const int w0 = threadIdx.x * per, w1 = min(W, w0 + per);
+    int cnt = 0;
+    for (int w = w0; w < w1; ++w) {
+        const int lo = w * 32;
+        const uint32_t valid = (lo + 32 <= n) ? 0xFFFFFFFFu : (lo >= n ? 0u : (0xFFFFFFFFu << (32 - (n - lo))));
+        const uint32_t m = __ldg(label + w) & valid;
+        mask[w] = m;
+        mask[W + w] = ~m & valid;
+        cnt += __popc(m);
+    }
+    int off = block_exclusive_scan(cnt, s_warp, &s_total);
+    int* out = xw.idx(0);
+    for (int w = w0; w < w1; ++w) {
+        uint32_t m = mask[w];
+        while (m) {
+            const int lz = __clz(m);
+            out[off++] = w * 32 + lz;
+            m &= ~(0x80000000u >> lz);
+        }
+    }
+    if (threadIdx.x == 0) {
+        XInfo* info = xw.info(0);
+        info->len[0][0] = s_total;
+        info->len[0][1] = info->len[1][0] = info->len[1][1] = 0;
+    }
+}
+
+// Genotype counts of the label's cases, and of the controls as the cohort's
+// minus those: one warp per SNP.
+__global__ void __launch_bounds__(256) label_marginals_kernel(const uint32_t* __restrict__ planes, int M, int W,
+                                                              const uint32_t* __restrict__ mask, int nc,
+                                                              const int* __restrict__ total, int* __restrict__ cases,
+                                                              int* __restrict__ controls) {
+    const int snp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (snp >= M) return;
+    const uint4* p0 = reinterpret_cast<const uint4*>(planes + (size_t)snp * 2 * W);
+    const uint4* p1 = p0 + W / 4;
+    const uint4* mk = reinterpret_cast<const uint4*>(mask);
+    int c0 = 0, c1 = 0;
+    for (int w = lane; w < W / 4; w += 32) {
+        const uint4 a = __ldg(p0 + w), b = __ldg(p1 + w), m = __ldg(mk + w);
+        c0 += __popc(a.x & m.x) + __popc(a.y & m.y) + __popc(a.z & m.z) + __popc(a.w & m.w);
+        c1 += __popc(b.x & m.x) + __popc(b.y & m.y) + __popc(b.z & m.z) + __popc(b.w & m.w);
+    }
+    c0 = __reduce_add_sync(0xFFFFFFFFu, c0);
+    c1 = __reduce_add_sync(0xFFFFFFFFu, c1);
+    if (lane < 3) {
+        const int v = lane == 0 ? c0 : lane == 1 ? c1 : nc - c0 - c1;
+        cases[lane * M + snp] = v;
+        controls[lane * M + snp] = total[lane * M + snp] - v;
+    }
+}
+
 // Regrouped operand rows for one X: row r, class c, segment s holds the e2m1
 // value bit(r, idx[c][s][k]) at packed sample position seg.kb0*256 + k (in
 // e2m1_word's order within each 32; zero past the segment's length up to its
@@ -560,8 +648,9 @@ static episdet_status prepare_stash(Workspace* w, int nz, int nseg, bool wide, C
 
 // Seed pass: bounds on one set per scoring thread over one tile per CTA pair
 // give a first search-wide threshold (the k-th best of some 38,000 sets that
-// are each the best of 28), so that from the first tile on only about one set
-// in a thousand is scored exactly and offered.
+// are each the best of 28), so that from the first tile on at most about one
+// set in a thousand is scored exactly and offered; the better seeds are levels
+// that the counting kernel tightens the threshold to as sets reach them.
 static episdet_status seed_threshold(Workspace* w, int inst, const CUtensorMap& ta, const CUtensorMap& tb,
                                      CountParams p, uint64_t* launches) {
     int pairs = 0;
@@ -572,7 +661,7 @@ static episdet_status seed_threshold(Workspace* w, int inst, const CUtensorMap& 
     p.seeds = (uint32_t*)w->seeds.p;
     st = launch_count(w, inst, ta, tb, p);
     if (st != EPISDET_OK) return st;
-    kth_key_kernel<<<1, kMergeBlockThreads, 0, w->st>>>(p.S, p.seeds, n);
+    seed_levels_kernel<<<1, kMergeBlockThreads, 0, w->st>>>(p.S, p.seeds, n);
     CHECK_LAUNCH();
     *launches += 2;
     return EPISDET_OK;
@@ -649,6 +738,85 @@ episdet_status tensor_pair_totals(Workspace* w, const uint32_t* d_planes, int M,
     return EPISDET_OK;
 }
 
+static episdet_status transpose_planes(Workspace* w, const DevData& D, int c, DevBuf* buf) {
+    const int rows = 2 * D.M, rwp = tt_row_words(rows);
+    CUDA_TRY(buf->ensure(sizeof(uint32_t) * (size_t)D.W[c] * 32 * rwp));
+    const int warps = (rwp / 8) * (D.W[c] / 8);
+    transpose_planes_kernel<<<(warps + kTtThreads / 32 - 1) / (kTtThreads / 32), kTtThreads, 0, w->st>>>(
+        D, c, (uint32_t*)buf->p, rows, rwp);
+    CHECK_LAUNCH();
+    return EPISDET_OK;
+}
+
+episdet_status tensor_label_cohort(Workspace* w, LabelCohort* c, bool validate) {
+    DevData D;
+    memset(&D, 0, sizeof(D));
+    D.M = c->M;
+    D.bits[0] = c->planes;
+    D.W[0] = c->W;
+    D.n[0] = c->n;
+    CUDA_TRY(w->perm_marg.ensure(sizeof(int) * 3 * (size_t)c->M));
+    CUDA_TRY(w->flag.ensure(sizeof(int) * 4));
+    CUDA_TRY(cudaMemsetAsync(w->flag.p, 0, sizeof(int) * 4, w->st));
+    cohort_marginals_kernel<<<(c->M + 7) / 8, 256, 0, w->st>>>(c->planes, c->M, c->n, c->W, (int*)w->perm_marg.p,
+                                                               (int*)w->flag.p);
+    CHECK_LAUNCH();
+    int bad = 0;
+    CUDA_TRY(cudaMemcpyAsync(&bad, w->flag.p, sizeof(int), cudaMemcpyDeviceToHost, w->st));
+    CUDA_TRY(cudaStreamSynchronize(w->st));
+    if (bad && validate)
+        return set_error(EPISDET_ERR_INVALID_INPUT, "input planes have overlapping genotype-0/1 planes");
+    episdet_status st = transpose_planes(w, D, 0, &w->perm_tt);
+    if (st != EPISDET_OK) return st;
+    CUDA_TRY(w->perm_tot.ensure(sizeof(float4) * (size_t)c->M * c->M));
+    st = tensor_pair_totals(w, c->planes, c->M, c->n, (float4*)w->perm_tot.p);  // ends with a synchronise
+    c->tt = (const uint32_t*)w->perm_tt.p;
+    c->marg = (const int*)w->perm_marg.p;
+    c->tot = (const float4*)w->perm_tot.p;
+    return st;
+}
+
+episdet_status tensor_label_rows(Workspace* w, const LabelCohort& c, const uint32_t* d_label, int nc, DevData* D,
+                                 uint64_t* launches) {
+    memset(D, 0, sizeof(*D));
+    D->M = c.M;
+    D->n[0] = nc;
+    D->n[1] = c.n - nc;
+    CUDA_TRY(w->perm_mask.ensure(sizeof(uint32_t) * 2 * (size_t)c.W));
+    uint32_t* mask = (uint32_t*)w->perm_mask.p;
+    for (int k = 0; k < 2; ++k) {
+        D->bits[k] = c.planes;
+        D->W[k] = c.W;
+        D->mask[k] = mask + (size_t)k * c.W;
+        CUDA_TRY(w->marg[k].ensure(sizeof(int) * 3 * (size_t)c.M));
+        D->marg[k] = (const int*)w->marg[k].p;
+    }
+    CUDA_TRY(w->tensor_flag.ensure(sizeof(int) * 4));
+    CUDA_TRY(cudaMemsetAsync(w->tensor_flag.p, 0, sizeof(int) * 4, w->st));
+    XWork xw;
+    xw.info_bytes = 256;
+    xw.stride = (xw.info_bytes + sizeof(int) * 4 * (size_t)c.n + 255) & ~size_t(255);
+    xw.max_n = c.n;
+    xw.x0 = 0;
+    CUDA_TRY(w->xinfo.ensure(xw.stride));
+    xw.base = (uint8_t*)w->xinfo.p;
+    label_lists_kernel<<<1, kXinfoThreads, 0, w->st>>>(d_label, c.n, c.W, xw, mask);
+    CHECK_LAUNCH();
+    label_marginals_kernel<<<(c.M + 7) / 8, 256, 0, w->st>>>(c.planes, c.M, c.W, mask, nc, c.marg, (int*)w->marg[0].p,
+                                                             (int*)w->marg[1].p);
+    CHECK_LAUNCH();
+    // Case operand rows: one member whose only segment is the cases.
+    const int rows = 2 * c.M, pitch = (episdet_class_words(nc) * 32 + kClassPad) / 2;
+    CUDA_TRY(w->frows.ensure((size_t)rows * pitch));
+    CmpOut co;
+    memset(&co, 0, sizeof(co));
+    co.out = (uint8_t*)w->frows.p;
+    regroup_kernel<<<kRgCtas * w->sms, kRgThreads, 0, w->st>>>(*D, xw, co, c.tt, c.tt, tt_row_words(rows), rows, pitch, 1);
+    CHECK_LAUNCH();
+    *launches += 3;
+    return EPISDET_OK;
+}
+
 episdet_status tensor_init_attributes() {
     for (int i = 0; i < kInstances; ++i)
         CUDA_TRY(cudaFuncSetAttribute(instance_at(i).kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -657,8 +825,9 @@ episdet_status tensor_init_attributes() {
 }
 
 // 2-way search: packed e2m1 rows of every SNP plane, one launch over the tiles
-// of the slab.  Label mode (w->label_tot): operand rows of the cases only; the
-// controls' cells come from the label-free pair totals.
+// of the slab.  Label mode (w->label_tot): operand rows of the cases only,
+// already in w->frows (tensor_label_rows); the controls' cells come from the
+// label-free pair totals.
 static episdet_status run_pairs(Workspace* w, const DevData& D, const episdet_options& o, int fb, int fe,
                                 CountParams& p, uint64_t* launches, bool progress) {
     const int M = D.M, Kc = D.W[0] * 32, Kn = D.W[1] * 32;
@@ -674,18 +843,23 @@ static episdet_status run_pairs(Workspace* w, const DevData& D, const episdet_op
         pair_tiles(M, a0, a1, nz, tiles);
     }
     const int inst = kIPairs + 2 * p.T.score + (narrow ? 1 : 0);
-    DevData Dp = D;
-    if (label) Dp.W[1] = 0;  // pack class 0 only
-    const int pitch = (Kc + kClassPad) / 2 + (label ? 0 : (Kn + kClassPad) / 2);
     CUtensorMap ta, tb;
-    episdet_status st = pack_rows(w, &w->frows, Dp, pitch, nz, &ta, &tb);
+    episdet_status st;
+    if (label) {
+        const int pitch = (episdet_class_words(D.n[0]) * 32 + kClassPad) / 2;
+        st = make_tmap(&ta, w->frows.p, (uint64_t)2 * M, (uint64_t)pitch, kCtaRows);
+        if (st == EPISDET_OK) st = make_tmap(&tb, w->frows.p, (uint64_t)2 * M, (uint64_t)pitch, nz);
+    } else {
+        st = pack_rows(w, &w->frows, D, (Kc + kClassPad) / 2 + (Kn + kClassPad) / 2, nz, &ta, &tb);
+        ++*launches;
+    }
     if (st != EPISDET_OK) return st;
     p.rt_ld = (M + 3) & ~3;
     CUDA_TRY(w->rtab.ensure(sizeof(float2) * 9 * (size_t)p.rt_ld));
     p.rt = (const float2*)w->rtab.p;
     marginal_rows_kernel<<<(M + 255) / 256, 256, 0, w->st>>>(D, (float2*)w->rtab.p, p.rt_ld, p.tab_off);
     CHECK_LAUNCH();
-    *launches += 2;
+    ++*launches;
     CUDA_TRY(w->tiles.ensure(sizeof(int2) * tiles.size()));
     CUDA_TRY(cudaMemcpyAsync(w->tiles.p, tiles.data(), sizeof(int2) * tiles.size(), cudaMemcpyHostToDevice, w->st));
     w->h2d += (int64_t)(sizeof(int2) * tiles.size());
@@ -925,10 +1099,8 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
     // Sample-major planes for the regrouping.
     const int rwp = tt_row_words(rows);
     for (int c = 0; c < 2; ++c) {
-        const int warps = (rwp / 8) * (D.W[c] / 8);
-        transpose_planes_kernel<<<(warps + kTtThreads / 32 - 1) / (kTtThreads / 32), kTtThreads, 0, w->st>>>(
-            D, c, (uint32_t*)w->planes_t[c].p, rows, rwp);
-        CHECK_LAUNCH();
+        st = transpose_planes(w, D, c, &w->planes_t[c]);
+        if (st != EPISDET_OK) return st;
         ++*launches;
     }
     // The regrouping reads the planes, their transposes and the marginals staged on st.
@@ -1012,12 +1184,6 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
             CUDA_TRY(timer_end(w));
             CUDA_TRY(cudaEventRecord(w->ev_tc[b], w->st));
             *launches += 1;
-            if (p.filter && (gi & (gi - 1)) == 0) {
-                // Tighten the search-wide threshold to the k-th best listed so far.
-                kth_key_kernel<<<1, kMergeBlockThreads, 0, w->st>>>(p.S, nullptr, 0);
-                CHECK_LAUNCH();
-                *launches += 1;
-            }
         }
     }
     if (w->timing) {

@@ -60,3 +60,57 @@ def test_more_ties_than_the_merge_holds(episdet, oracle, score):
 def test_autotune_keeps_the_answer(episdet, oracle):
     check(episdet, oracle, 3, 120, 2000, 2100, "k2", 200, flags=(episdet.FLAG_AUTOTUNE, 0))
     assert episdet.tuned_stage(3, "k2", 2000, 2100) in (0, 1)
+
+
+def test_permutations_device_labels_and_unaligned_planes(episdet, oracle):
+    """Label mode takes labels and planes of either memory; planes that are not
+    16-byte aligned go through the per-label split.  Same answers."""
+    import numpy as np
+    import torch
+
+    n, M, nc, nl = 2085, 150, 700, 3
+    planes = episdet.generate_cohort(77, M, n)
+    labels = episdet.generate_labels(78, n, nc, nl)
+    want = []
+    for lab in labels:
+        a, b, na, nb = oracle.split_by_label(planes, n, lab)
+        want.append(oracle.search(a, b, na, nb, order=2, score="k2", top_k=40))
+    dev = torch.from_numpy(planes.view(np.int32)).cuda()
+    shifted = torch.zeros(dev.numel() + 1, dtype=torch.int32, device="cuda")
+    shifted[1:] = dev.flatten()
+    off = shifted[1:].view(dev.shape)
+    dl = torch.from_numpy(labels.view(np.int32)).cuda()
+    torch.cuda.synchronize()
+    assert off.data_ptr() % 16 == 4
+    for p, q in ((planes, labels), (dev, dl), (off, dl)):
+        for r, o in zip(episdet.search_perm(p, n, q, order=2, score="k2", top_k=40), want):
+            assert_same(r, o, 40)
+
+
+def test_permutations_reject_overlapping_planes(episdet):
+    n, M = 1500, 20
+    planes = episdet.generate_cohort(5, M, n)
+    labels = episdet.generate_labels(6, n, 600, 2)
+    bad = planes.copy()
+    bad[3, 0, 1] |= 0x10
+    bad[3, 1, 1] |= 0x10
+    with pytest.raises(episdet.EpisdetError) as e:
+        episdet.search_perm(bad, n, labels, top_k=8)
+    assert e.value.name == "EPISDET_ERR_INVALID_INPUT"
+    empty = labels.copy()
+    empty[1] = 0
+    with pytest.raises(episdet.EpisdetError) as e:
+        episdet.search_perm(planes, n, empty, top_k=8)
+    assert e.value.name == "EPISDET_ERR_INVALID_ARGUMENT" and "label 1" in str(e.value)
+
+
+@pytest.mark.parametrize("M,n", [(1, 2), (7, 1025), (8, 33000), (17, 70001)])
+def test_binarize_groups_and_chunks(episdet, oracle, M, n):
+    import numpy as np
+
+    rng = np.random.default_rng(M)
+    g = rng.integers(0, 3, size=(M, n)).astype(np.uint8)
+    flags = rng.random(n) < 0.3
+    flags[0], flags[-1] = True, False
+    cases, controls, nc, nn = episdet.binarize(g, flags)
+    assert np.array_equal(cases, oracle.pack(g[:, flags])) and np.array_equal(controls, oracle.pack(g[:, ~flags]))
