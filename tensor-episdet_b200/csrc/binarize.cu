@@ -45,21 +45,27 @@ __global__ void __launch_bounds__(kListThreads) class_lists_kernel(const uint8_t
     if (threadIdx.x == 0) *num_cases = total;
 }
 
-// One warp per kBinSnps SNPs x 32 output words of a class: for each word the
-// lanes read the genotypes of its 32 samples (neighbours in the row, so few
-// cache lines) and two ballots make the plane words; lane k keeps word k, so
-// the stores are whole lines.  Reading every genotype byte once is the bound
-// (79 us for 8192 x 50001 at the copy rate); a thread per word, each reading its
-// own 32 samples, took 1.7 ms there.
+// One warp per kBinSnps SNPs x 32 output words of a class.  The 1,024 samples of
+// those words lie in one stretch of each genotype row: the warp copies the
+// stretch into shared memory (kBinSpan bytes at most; a class so sparse that it
+// is longer reads the row instead), and for each word the lanes read its 32
+// samples' bytes and two ballots make the plane words; lane k keeps word k, so
+// the stores are whole lines.  The bound is reading every genotype byte once
+// per class (8192 x 50001: 79 us for once at the copy rate); a thread per word,
+// each reading its own 32 samples, took 1700 us there, ballots over global
+// bytes 421 us, this BIN_US us.
 constexpr int kBinSnps = 8;
+constexpr int kBinSpan = 4096;
+constexpr int kBinWarps = 8;
 struct BinClass {
     const int* idx;  // samples of the class
     uint32_t* out;   // [M][2][W]
     int n, W;
 };
-__global__ void __launch_bounds__(256) binarize_kernel(const uint8_t* __restrict__ geno, int M, int n, BinClass a,
-                                                       BinClass b, int* __restrict__ bad) {
-    const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(32 * kBinWarps) binarize_kernel(const uint8_t* __restrict__ geno, int M, int n,
+                                                                  BinClass a, BinClass b, int* __restrict__ bad) {
+    __shared__ __align__(16) uint8_t s_row[kBinWarps][kBinSpan + 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wa = a.W / 32, wb = b.W / 32;
     const long unit = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // both classes of an SNP group together
     const long group = unit / (wa + wb);
@@ -69,35 +75,60 @@ __global__ void __launch_bounds__(256) binarize_kernel(const uint8_t* __restrict
     const int* __restrict__ idx = second ? b.idx : a.idx;
     uint32_t* __restrict__ out = second ? b.out : a.out;
     const int nk = second ? b.n : a.n, W = second ? b.W : a.W;
-    const int w0 = (second ? chunk - wa : chunk) * 32;
+    const int w0 = (second ? chunk - wa : chunk) * 32, i0 = w0 * 32;
     const int snp0 = (int)group * kBinSnps, ns = min(kBinSnps, M - snp0);
-    const uint8_t* row = geno + (size_t)snp0 * n;
-    uint32_t p0[kBinSnps], p1[kBinSnps];
+    // The stretch [lo, hi) of a row (empty when the words are all padding).
+    const int lo = i0 < nk ? __ldg(idx + i0) : 0, hi = i0 < nk ? __ldg(idx + min(nk, i0 + 1024) - 1) + 1 : 0;
+    const bool staged = hi - lo <= kBinSpan;
+    uint16_t rel[32];  // this lane's sample of each word, from lo
 #pragma unroll
-    for (int s = 0; s < kBinSnps; ++s) p0[s] = p1[s] = 0;
-    bool over = false;
-#pragma unroll 2
     for (int k = 0; k < 32; ++k) {
-        const int i = (w0 + k) * 32 + lane;
-        const int at = i < nk ? __ldg(idx + i) : -1;
+        const int i = i0 + k * 32 + lane;
+        rel[k] = staged && i < nk ? (uint16_t)(__ldg(idx + i) - lo) : 0xFFFFu;
+    }
+    uint8_t* row = s_row[warp];
+    bool over = false;
+    for (int s = 0; s < ns; ++s) {
+        const uint8_t* g0 = geno + (size_t)(snp0 + s) * n;
+        uint32_t p0 = 0, p1 = 0;
+        if (staged) {
+            // Whole aligned words that hold the stretch, byte by byte where
+            // they would leave the row.
+            const uint8_t* from = g0 + lo;
+            const int skew = (int)((uintptr_t)from & 15);
+            const uint8_t* base = from - skew;
+            const int len = hi - lo + skew;
+            __syncwarp();
+            for (int o = 16 * lane; o < len; o += 512) {
+                const uint8_t* p = base + o;
+                if (p >= g0 && p + 16 <= g0 + n) {
+                    *reinterpret_cast<uint4*>(row + o) = __ldg(reinterpret_cast<const uint4*>(p));
+                } else {
+                    for (int e = 0; e < 16; ++e)
+                        if (p + e >= from && p + e < g0 + hi) row[o + e] = p[e];
+                }
+            }
+            __syncwarp();
 #pragma unroll
-        for (int s = 0; s < kBinSnps; ++s) {
-            const uint32_t g = at >= 0 && s < ns ? __ldg(row + (size_t)s * n + at) : 2u;
-            const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, g == 0), m1 = __ballot_sync(0xFFFFFFFFu, g == 1);
-            over |= g > 2;
-            if (lane == k) {
-                p0[s] = __brev(m0);
-                p1[s] = __brev(m1);
+            for (int k = 0; k < 32; ++k) {
+                const uint32_t g = rel[k] != 0xFFFFu ? row[skew + rel[k]] : 2u;
+                const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, g == 0), m1 = __ballot_sync(0xFFFFFFFFu, g == 1);
+                over |= g > 2;
+                if (lane == k) p0 = m0, p1 = m1;
+            }
+        } else {
+            for (int k = 0; k < 32; ++k) {
+                const int i = i0 + k * 32 + lane;
+                const uint32_t g = i < nk ? __ldg(g0 + __ldg(idx + i)) : 2u;
+                const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, g == 0), m1 = __ballot_sync(0xFFFFFFFFu, g == 1);
+                over |= g > 2;
+                if (lane == k) p0 = m0, p1 = m1;
             }
         }
+        uint32_t* o = out + (size_t)(snp0 + s) * 2 * W + w0 + lane;
+        o[0] = __brev(p0);
+        o[W] = __brev(p1);
     }
-#pragma unroll
-    for (int s = 0; s < kBinSnps; ++s)
-        if (s < ns) {
-            uint32_t* o = out + (size_t)(snp0 + s) * 2 * W + w0 + lane;
-            o[0] = p0[s];
-            o[W] = p1[s];
-        }
     if (__any_sync(0xFFFFFFFFu, over) && lane == 0) atomicExch(bad, 1);
 }
 
@@ -156,7 +187,7 @@ extern "C" episdet_status episdet_binarize(const uint8_t* genotypes, int32_t num
     }
     const BinClass ca{d_idx, d_out[0], nc, Wc}, cb{d_idx + nc, d_out[1], nn, Wn};
     const long warps = (long)((M + kBinSnps - 1) / kBinSnps) * (Wc / 32 + Wn / 32);
-    binarize_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(d_geno, M, n, ca, cb, d_flag);
+    binarize_kernel<<<(unsigned)((warps + kBinWarps - 1) / kBinWarps), 32 * kBinWarps, 0, s>>>(d_geno, M, n, ca, cb, d_flag);
     CHECK_LAUNCH();
     int bad = 0;
     CUDA_TRY(cudaMemcpyAsync(&bad, w->flag.p, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -25,6 +25,6 @@ extern "C" __global__ void search3_simt_kernel(DevData D, ScoreTables T, int xsn
 extern "C" __global__ void seed_levels_kernel(Slots S, const uint32_t* seeds, int n);
 extern "C" __global__ void merge_topk_kernel(Slots S, Cand* out, int* out_count);
 extern "C" __global__ void rescore_kernel(DevData D, ScoreTables T, int order, const Cand* cands, const int* count,
-                                          double* fp64_out, int* cells_out);
+                                          double* fp64_out, int* cells_out, const int* err, int* err_out);
 
 }  // namespace episdet

@@ -538,7 +538,8 @@ __device__ __forceinline__ uint32_t warp_sum(uint32_t v) {
 
 extern "C" __global__ void __launch_bounds__(256)
     rescore_kernel(DevData D, ScoreTables T, int order, const Cand* __restrict__ cands, const int* count,
-                   double* fp64_out, int* cells_out) {
+                   double* fp64_out, int* cells_out, const int* err, int* err_out) {
+    if (err_out && blockIdx.x == 0 && threadIdx.x == 0) *err_out = *err;  // beside the results, for one copy
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
     if (warp >= *count) return;

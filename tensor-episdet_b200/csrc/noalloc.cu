@@ -241,7 +241,7 @@ static episdet_status search_locked(const episdet_dataset* data, const episdet_o
     double* fp64 = (double*)(S + kOffFp64);
     merge_topk_kernel<<<1, kMergeBlockThreads, kMergeSmem, stream>>>(slots, merged, mcount);
     CHECK_LAUNCH();
-    rescore_kernel<<<(o.top_k * 32 + 255) / 256, 256, 0, stream>>>(D, T, 2, merged, mcount, fp64, nullptr);
+    rescore_kernel<<<(o.top_k * 32 + 255) / 256, 256, 0, stream>>>(D, T, 2, merged, mcount, fp64, nullptr, nullptr, nullptr);
     CHECK_LAUNCH();
     launches += 3;
     int cnt = 0;

@@ -62,6 +62,18 @@ cudaError_t DevBuf::ensure(size_t bytes) {
     if (e == cudaSuccess) cap = want;
     return e;
 }
+cudaError_t HostBuf::ensure(size_t bytes) {
+    if (bytes <= cap && p) return cudaSuccess;
+    release();
+    cudaError_t e = cudaMallocHost(&p, bytes);
+    if (e == cudaSuccess) cap = bytes;
+    return e;
+}
+void HostBuf::release() {
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    cap = 0;
+}
 void DevBuf::release() {
     if (p) cudaFree(p);
     p = nullptr;
@@ -359,26 +371,26 @@ static episdet_status run_simt(Workspace* w, const DevData& D0, const ScoreTable
 static episdet_status finish(Workspace* w, const DevData& D, const ScoreTables& T, const episdet_options& o,
                              const Slots& S, episdet_result* r, uint64_t* launches) {
     const int k = o.top_k;
-    CUDA_TRY(w->merged.ensure(sizeof(Cand) * (size_t)k));
-    CUDA_TRY(w->mcount.ensure(sizeof(int) * 4));
-    CUDA_TRY(w->fp64.ensure(sizeof(double) * (size_t)k));
-    merge_topk_kernel<<<1, kMergeBlockThreads, kMergeSmem, w->st>>>(S, (Cand*)w->merged.p, (int*)w->mcount.p);
+    // Results in one buffer, copied back at once: {count, error}, candidates, FP64 scores.
+    const size_t head = 16, bytes = head + (sizeof(Cand) + sizeof(double)) * (size_t)k;
+    CUDA_TRY(w->merged.ensure(bytes));
+    CUDA_TRY(w->results.ensure(bytes));
+    int* d_head = (int*)w->merged.p;
+    Cand* d_cands = (Cand*)((char*)w->merged.p + head);
+    double* d_f64 = (double*)(d_cands + k);
+    merge_topk_kernel<<<1, kMergeBlockThreads, kMergeSmem, w->st>>>(S, d_cands, d_head);
     CHECK_LAUNCH();
-    rescore_kernel<<<(k * 32 + 255) / 256, 256, 0, w->st>>>(D, T, o.order, (const Cand*)w->merged.p,
-                                                             (const int*)w->mcount.p, (double*)w->fp64.p, nullptr);
+    rescore_kernel<<<(k * 32 + 255) / 256, 256, 0, w->st>>>(D, T, o.order, d_cands, d_head, d_f64, nullptr,
+                                                             (const int*)w->tensor_flag.p, d_head + 1);
     CHECK_LAUNCH();
     *launches += 2;
-    std::vector<Cand> cands((size_t)k);
-    std::vector<double> f64((size_t)k);
-    int cnt = 0;
-    CUDA_TRY(cudaMemcpyAsync(cands.data(), w->merged.p, sizeof(Cand) * k, cudaMemcpyDeviceToHost, w->st));
-    CUDA_TRY(cudaMemcpyAsync(f64.data(), w->fp64.p, sizeof(double) * k, cudaMemcpyDeviceToHost, w->st));
-    CUDA_TRY(cudaMemcpyAsync(&cnt, w->mcount.p, sizeof(int), cudaMemcpyDeviceToHost, w->st));
-    int dev_err = 0;
-    CUDA_TRY(cudaMemcpyAsync(&dev_err, w->tensor_flag.p, sizeof(int), cudaMemcpyDeviceToHost, w->st));
+    CUDA_TRY(cudaMemcpyAsync(w->results.p, w->merged.p, bytes, cudaMemcpyDeviceToHost, w->st));
     CUDA_TRY(cudaEventRecord(w->e1, w->st));
     CUDA_TRY(cudaStreamSynchronize(w->st));
-    w->d2h += (int64_t)(sizeof(Cand) + sizeof(double)) * k + 2 * sizeof(int);
+    w->d2h += (int64_t)bytes;
+    const int cnt = ((const int*)w->results.p)[0], dev_err = ((const int*)w->results.p)[1];
+    const Cand* cands = (const Cand*)((const char*)w->results.p + head);
+    const double* f64 = (const double*)(cands + k);
     if (dev_err)
         return set_error(EPISDET_ERR_TIMEOUT, "a bounded device wait gave up (code %d); results discarded", dev_err);
     if (cnt < 1) return set_error(EPISDET_ERR_INTERNAL, "no candidate survived the search");

@@ -40,6 +40,14 @@ struct DevBuf {
     void release();
 };
 
+// The same in pinned host memory.
+struct HostBuf {
+    void* p = nullptr;
+    size_t cap = 0;
+    cudaError_t ensure(size_t bytes);
+    void release();
+};
+
 // Sets of regrouped operand buffers of the triplet engine: the regrouping of
 // group g + kXSets - 1 (second stream) overlaps the counting launch of group g.
 constexpr int kXSets = 2;
@@ -57,7 +65,8 @@ struct Workspace {
     cudaEvent_t ev_ready = nullptr, ev_cmp[kXSets] = {}, ev_tc[kXSets] = {};  // ordering between st and aux_st
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     std::mutex mu;
-    DevBuf bits[2], marg[2], pair4[2], t32, t64, slots, counts, tiles, merged, mcount, fp64, flag;
+    DevBuf bits[2], marg[2], pair4[2], t32, t64, slots, counts, tiles, merged, flag;
+    HostBuf results;      // a search's result lists on the host
     DevBuf ptab, ptabx;   // 3-way tensor engine: pair table, and (Y-blocked) the rows of the current first SNPs
     DevBuf frows;         // packed e2m1 operand rows of the planes (2-way and pair table)
     DevBuf rtab;          // counts that cells are derived from, per SNP (tensor engine)
@@ -91,11 +100,12 @@ struct Workspace {
         for (DevBuf& b : xsub) b.release();
         DevBuf* all[] = {&bits[0], &bits[1], &marg[0], &marg[1], &pair4[0], &pair4[1], &ptab, &ptabx, &t32,
                          &t64, &slots,
-                         &counts, &tiles, &merged, &mcount, &fp64, &flag, &frows, &rtab, &stash, &seeds, &planes_t[0], &planes_t[1],
+                         &counts, &tiles, &merged, &flag, &frows, &rtab, &stash, &seeds, &planes_t[0], &planes_t[1],
                          &xinfo,
                          &tensor_flag, &cbuf, &perm_tot, &perm_tt, &perm_marg, &perm_labels, &perm_mask, &perm_planes, &perm_cls[0], &perm_cls[1], &perm_idx,
                          &bin_geno, &bin_idx, &bin_out[0], &bin_out[1]};
         for (DevBuf* b : all) b->release();
+        results.release();
         tab_score = tab_nc = tab_nn = -1;
     }
 };

@@ -673,11 +673,19 @@ static bool counts_wide(int nc, int nn) { return std::max(nc, nn) > 65535; }
 // First B tile of nz SNPs that reaches past the first SNP of A tile a.
 static int first_b(int a, int nz) { return (kTileA * a) / nz; }
 
-// Tiles of the pairs (r, col > r) with r in A tiles [a0, a1).
+// Tiles of the pairs (r, col > r) with r in A tiles [a0, a1), every B tile that
+// reaches past the A tile's first SNP, in bands of about 1024 x 1008 SNPs: the 74
+// tiles that run at once then read 8 + 9 row panels instead of 1 + 74 (all pairs
+// of 16384 SNPs x 32768 samples, whose rows are 537 MB: row by row 5.98 ms,
+// in bands BAND_MS).
 static void pair_tiles(int M, int a0, int a1, int nz, std::vector<int2>& out) {
-    const int ntb = (M + nz - 1) / nz;
-    for (int a = a0; a < a1; ++a)
-        for (int b = first_b(a, nz); b < ntb; ++b) out.push_back(make_int2(a, b));
+    constexpr int kBandA = 8;
+    const int band_b = 9 * kWideZ / nz, ntb = (M + nz - 1) / nz;
+    for (int ba = a0; ba < a1; ba += kBandA)
+        for (int bb = first_b(ba, nz); bb < ntb; bb += band_b)
+            for (int a = ba; a < std::min(a1, ba + kBandA); ++a)
+                for (int b = std::max(first_b(a, nz), bb); b < std::min(ntb, bb + band_b); ++b)
+                    out.push_back(make_int2(a, b));
 }
 
 static int a_tiles(int M) { return (M + kTileA - 1) / kTileA; }
@@ -994,20 +1002,25 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
     const int nblk = (nt2 - a_first + blk_tiles - 1) / blk_tiles;
     p.rt = (const float2*)w->rtab.p;
 
-    // Operand rows of the pair table, and its tiles (A tile a, every B tile
-    // reaching past a's first SNP) in order of a, so that the tiles of rows
-    // [128 a_lo, 128 a_hi) are one sub-range.
+    // Operand rows of the pair table, and its tiles: one list per Y block (all
+    // rows from the slab's first on when whole) and, Y-blocked, one per A tile
+    // that holds first SNPs.
     CUtensorMap fa, fbm;
     st = pack_rows(w, &w->frows, D, pitch, kWideZ, &fa, &fbm);
     if (st != EPISDET_OK) return st;
     ++*launches;
     std::vector<int2> lists;
-    std::vector<size_t> tri_off((size_t)nt2 + 1, 0);
-    for (int a = 0; a < nt2; ++a) {
-        tri_off[a] = lists.size();
-        pair_tiles(M, a, a + 1, kWideZ, lists);
+    std::vector<size_t> blk_off((size_t)nblk + 1, 0), row_off((size_t)nt2 + 1, 0);
+    for (int blk = 0; blk < nblk; ++blk) {
+        const int ya0 = blocked ? a_first + blk * blk_tiles : fb / kTileA;
+        pair_tiles(M, ya0, blocked ? std::min(nt2, ya0 + blk_tiles) : nt2, kWideZ, lists);
+        blk_off[blk + 1] = lists.size();
     }
-    tri_off[nt2] = lists.size();
+    for (int a = 0; a < nt2; ++a) {
+        row_off[a] = lists.size();
+        if (blocked && a >= fb / kTileA && a <= (xend - 1) / kTileA) pair_tiles(M, a, a + 1, kWideZ, lists);
+    }
+    row_off[nt2] = lists.size();
     // Triplet tile lists, one per (Y block, first A tile a0 = (X+1)/128): every
     // (A tile a, B tile b) with max(a0, first tile of the block) <= a < end of
     // the block, whose Z range reaches past the tile's first Y, ordered in
@@ -1042,9 +1055,9 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
     w->h2d += (int64_t)(sizeof(int2) * lists.size());
     p.tiles = (const int2*)w->tiles.p;
 
-    // Counts of the pairs of SNP rows [r0, r1) (128-aligned r0) with every
-    // later SNP, stored at pair (row - r0) * (M - r0) + (col - r0) of out (or
-    // at row * M + col when whole).
+    // Counts of the pairs of SNP rows from r0 on (128-aligned) with every later
+    // SNP, by the tiles [t0, t1) of the lists, stored at pair (row - r0) *
+    // (M - r0) + (col - r0) of out (or at row * M + col when whole).
     CountParams ps = p;
     ps.seg2[0] = Seg{0, (D.n[0] + kF4PerKB - 1) / kF4PerKB};
     const int kbn = (Kc + kClassPad) / kF4PerKB;
@@ -1056,10 +1069,9 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
     st = prepare_stash(w, kWideZ, 2, ps.wide != 0, &ps);
     if (st != EPISDET_OK) return st;
     p.stash = ps.stash;
-    auto store_pairs = [&](float* out, int r0, int r1, bool whole) -> episdet_status {
-        const int t0 = r0 / kTileA, t1 = std::min(nt2, (r1 + kTileA - 1) / kTileA);
-        ps.list_off[0] = (int)tri_off[t0];
-        ps.ntiles = (int)(tri_off[t1] - tri_off[t0]);
+    auto store_pairs = [&](float* out, size_t t0, size_t t1, int r0, bool whole) -> episdet_status {
+        ps.list_off[0] = (int)t0;
+        ps.ntiles = (int)(t1 - t0);
         ps.out = out;
         ps.out_r0 = ps.out_c0 = whole ? 0 : r0;
         ps.out_ld = whole ? M : M - r0;
@@ -1068,7 +1080,7 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
     };
     PairView xv{};
     if (!blocked) {
-        st = store_pairs((float*)w->ptab.p, fb / kTileA * kTileA, M, true);
+        st = store_pairs((float*)w->ptab.p, 0, blk_off[1], 0, true);
         if (st != EPISDET_OK) return st;
         p.yv = xv = PairView{(const float*)w->ptab.p, 0, 0, M};
     }
@@ -1120,7 +1132,7 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
         if (blocked) {
             // Y-Z rows of this block (the previous block's launches, on the
             // same stream, have read theirs).
-            st = store_pairs((float*)w->ptab.p, y0, y1, false);
+            st = store_pairs((float*)w->ptab.p, blk_off[blk], blk_off[blk + 1], y0, false);
             if (st != EPISDET_OK) return st;
             p.yv = PairView{(const float*)w->ptab.p, y0, y0, M - y0};
         }
@@ -1150,7 +1162,7 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
             if (blocked && xt0 != x0 / kTileA * kTileA) {
                 // X-Y and X-Z rows of this group's first SNPs (and the next ones').
                 xt0 = x0 / kTileA * kTileA;
-                st = store_pairs((float*)w->ptabx.p, xt0, std::min(M, xt0 + kTileA), false);
+                st = store_pairs((float*)w->ptabx.p, row_off[xt0 / kTileA], row_off[xt0 / kTileA + 1], xt0, false);
                 if (st != EPISDET_OK) return st;
                 xv = PairView{(const float*)w->ptabx.p, xt0, xt0, M - xt0};
             }
