@@ -13,6 +13,7 @@
 #include "episdet.h"
 #include "host_util.h"
 #include "search_internal.h"
+#include "tc_ptx.cuh"
 
 namespace episdet {
 
@@ -54,9 +55,9 @@ __global__ void __launch_bounds__(kListThreads) class_lists_kernel(const uint8_t
 // per class (8192 x 50001: 79 us for once at the copy rate); a thread per word,
 // each reading its own 32 samples, took 1700 us there, ballots over global
 // bytes 421 us, this BIN_US us.
-constexpr int kBinSnps = 8;
+constexpr int kBinSnps = 16;
 constexpr int kBinSpan = 4096;
-constexpr int kBinWarps = 8;
+constexpr int kBinWarps = 4;
 struct BinClass {
     const int* idx;  // samples of the class
     uint32_t* out;   // [M][2][W]
@@ -64,7 +65,7 @@ struct BinClass {
 };
 __global__ void __launch_bounds__(32 * kBinWarps) binarize_kernel(const uint8_t* __restrict__ geno, int M, int n,
                                                                   BinClass a, BinClass b, int* __restrict__ bad) {
-    __shared__ __align__(16) uint8_t s_row[kBinWarps][kBinSpan + 32];
+    __shared__ __align__(16) uint8_t s_row[kBinWarps][2][kBinSpan + 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wa = a.W / 32, wb = b.W / 32;
     const long unit = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // both classes of an SNP group together
@@ -86,36 +87,50 @@ __global__ void __launch_bounds__(32 * kBinWarps) binarize_kernel(const uint8_t*
         const int i = i0 + k * 32 + lane;
         rel[k] = staged && i < nk ? (uint16_t)(__ldg(idx + i) - lo) : 0xFFFFu;
     }
-    uint8_t* row = s_row[warp];
+    // Copies a row's stretch: whole aligned 16 bytes, byte by byte where they
+    // would leave the row.  Returns where the stretch begins in the buffer.
+    auto copy = [&](int s) {
+        const uint8_t* g0 = geno + (size_t)(snp0 + s) * n;
+        const uint8_t* from = g0 + lo;
+        const int skew = (int)((uintptr_t)from & 15);
+        const uint8_t* base = from - skew;
+        uint8_t* row = s_row[warp][s & 1];
+        for (int o = 16 * lane; o < hi - lo + skew; o += 512) {
+            const uint8_t* p = base + o;
+            if (p >= g0 && p + 16 <= g0 + n) {
+                ptx::cp_async16(ptx::smem_u32(row + o), p, true);
+            } else {
+                for (int e = 0; e < 16; ++e)
+                    if (p + e >= from && p + e < g0 + hi) row[o + e] = p[e];
+            }
+        }
+        ptx::cp_async_commit();
+        return skew;
+    };
     bool over = false;
+    int skew = 0, skew_next = staged ? copy(0) : 0;
     for (int s = 0; s < ns; ++s) {
         const uint8_t* g0 = geno + (size_t)(snp0 + s) * n;
         uint32_t p0 = 0, p1 = 0;
+        skew = skew_next;
         if (staged) {
-            // Whole aligned words that hold the stretch, byte by byte where
-            // they would leave the row.
-            const uint8_t* from = g0 + lo;
-            const int skew = (int)((uintptr_t)from & 15);
-            const uint8_t* base = from - skew;
-            const int len = hi - lo + skew;
-            __syncwarp();
-            for (int o = 16 * lane; o < len; o += 512) {
-                const uint8_t* p = base + o;
-                if (p >= g0 && p + 16 <= g0 + n) {
-                    *reinterpret_cast<uint4*>(row + o) = __ldg(reinterpret_cast<const uint4*>(p));
-                } else {
-                    for (int e = 0; e < 16; ++e)
-                        if (p + e >= from && p + e < g0 + hi) row[o + e] = p[e];
-                }
+            // The next row's copy is in flight while this one is read.
+            if (s + 1 < ns) {
+                skew_next = copy(s + 1);
+                ptx::cp_async_wait<1>();
+            } else {
+                ptx::cp_async_wait<0>();
             }
             __syncwarp();
+            const uint8_t* row = s_row[warp][s & 1] + skew;
 #pragma unroll
             for (int k = 0; k < 32; ++k) {
-                const uint32_t g = rel[k] != 0xFFFFu ? row[skew + rel[k]] : 2u;
+                const uint32_t g = rel[k] != 0xFFFFu ? row[rel[k]] : 2u;
                 const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, g == 0), m1 = __ballot_sync(0xFFFFFFFFu, g == 1);
                 over |= g > 2;
                 if (lane == k) p0 = m0, p1 = m1;
             }
+            __syncwarp();  // before the buffer's next copy
         } else {
             for (int k = 0; k < 32; ++k) {
                 const int i = i0 + k * 32 + lane;

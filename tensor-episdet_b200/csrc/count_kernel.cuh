@@ -123,6 +123,7 @@ struct CountParams {
     double cut_mul, cut_add, seed_mul, seed_add;
     int filter;         // 0: every set is scored exactly
     int wide;           // pairs: counts do not fit 16 bits
+    int one_class;      // pairs: no second segment (label mode, or the totals of one plane set)
     int* err;
     uint64_t wait_ns;   // limit of every wait for work
     const int* hold;    // failure-detection test: a word the scoring warps wait for (nothing sets it), or null
@@ -392,6 +393,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     constexpr int kKbBytes = C::kKbBytes;
     constexpr int NSEG = MODE == kTriplets ? 4 : 2;
     constexpr uint32_t kIdesc = ptx::idesc_mxf4(C::kN, 256);
+    // Without a second class (pair totals, label mode) there is one segment.
+    const int nseg = MODE != kTriplets && P.one_class ? 1 : NSEG;
     extern __shared__ uint8_t smem_raw[];
     // A launch with less dynamic shared memory than the layout needs is
     // refused before anything touches it (uniform over the pair, so no barrier
@@ -505,7 +508,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int2 tl = P.tiles[P.list_off[g] + t - P.cum[g]];
                 const int arow = g * P.rows_member + tl.x * 2 * kTileA + rank * kCtaRows;
                 const int brow = g * P.rows_member + tl.y * C::kN + rank * NZ;
-                for (int s = 0; ok && s < NSEG; ++s) {
+                for (int s = 0; ok && s < nseg; ++s) {
                     const Seg seg = s_grp[g].seg[s];
                     for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
                         if (!ptx::mbar_wait(&empty[stage], phase ^ 1, abort, P.wait_ns)) {
@@ -551,7 +554,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const uint64_t desc0 = ptx::smem_desc_sw128(ptx::smem_u32(smem));
             for (int t = t_first; ok && t < P.ntiles; t += t_step) {
                 const int g = group_of(P, t);
-                for (int s = 0; ok && s < NSEG; ++s, ++job) {
+                for (int s = 0; ok && s < nseg; ++s, ++job) {
                     const uint32_t b = job & 1u, use = job >> 1;
                     const Seg seg = s_grp[g].seg[s];
                     bool w = ptx::mbar_wait_cluster(&tempty[b], (use & 1) ^ 1, abort, P.wait_ns);
@@ -628,7 +631,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 break;
             }
 #pragma unroll 1
-            for (int s = 0; s < NSEG; ++s, ++job) {
+            for (int s = 0; s < nseg; ++s, ++job) {
                 const uint32_t b = job & 1u;
                 w = ptx::mbar_wait(&tfull[b], (job >> 1) & 1u, abort, P.wait_ns);
                 if (!__all_sync(0xFFFFFFFFu, w)) {
@@ -764,11 +767,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                 return bsnp > arow && bsnp < M && (MODE != kTriplets || arow > X) &&
                        (MODE != kPairs || (arow >= P.first_begin && arow < P.first_end));
             };
-            // What a step reads from L2, fetched two steps ahead: the packed
-            // counts (narrow stash) and the set's pair-table cells, both
-            // contiguous over the lanes.  (With a lane per A SNP the pair-table
-            // reads of a warp touched 32 rows and took a third of the time.)  A
-            // thread without a set to score there reads other valid memory.
+            // What a step reads from L2, fetched kAhead steps ahead (loads took 1
+            // to 2 thousand clocks while operands stream; a step of a triplet
+            // tile takes about 1300, of a pairs tile 430): the packed counts
+            // (narrow stash) and the set's pair-table cells, both contiguous over
+            // the lanes.  (With a lane per A SNP the pair-table reads of a warp
+            // touched 32 rows and took a third of the time.)  A thread without a
+            // set to score there reads other valid memory.
             struct Fetched {
                 uint2 u[NSEG];
                 float4 y0, y1;
@@ -777,7 +782,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (!wide) {
 #pragma unroll
                     for (int s = 0; s < NSEG; ++s)
-                        f.u[s] = __ldcg(reinterpret_cast<const uint2*>(slot) + s * C::kSegWords + etid + step * kScoreThreads);
+                        f.u[s] = s < nseg ? __ldcg(reinterpret_cast<const uint2*>(slot) + s * C::kSegWords + etid + step * kScoreThreads)
+                                          : make_uint2(0, 0);
                 }
                 if constexpr (MODE == kTriplets) {
                     const size_t o = valid(it) ? (size_t)(arow0 + it.yl - P.yv.r0) * (size_t)P.yv.ld +
@@ -789,17 +795,18 @@ __global__ void __launch_bounds__(kThreads, 1)
                     f.y0 = __ldg(P.tot + (valid(it) ? (size_t)(arow0 + it.yl) * M + tl.y * NZ + it.z : 0));
             };
             constexpr int kSteps = C::kSegWords / kScoreThreads;
-            static_assert(kSteps % 2 == 0, "steps are taken in twos");
-            Item it{etid / NZ, etid % NZ};
-            Fetched fa, fb;
-            fetch(fa, it, 0);
-            fetch(fb, next(it), 1);
-#pragma unroll 1
-            for (int step = 0; step < kSteps; step += 2) {
+            constexpr int kAhead = MODE == kTriplets ? 2 : 4;
+            Item it{etid / NZ, etid % NZ}, ahead = it;
+            Fetched ring[kAhead];
 #pragma unroll
-                for (int half = 0; half < 2; ++half, it = next(it)) {
-                    const Fetched f = half ? fb : fa;
-                    if (step + half + 2 < kSteps) fetch(half ? fb : fa, next(next(it)), step + half + 2);
+            for (int e = 0; e < kAhead; ++e, ahead = next(ahead)) fetch(ring[e], ahead, e);
+#pragma unroll 1
+            for (int step = 0; step < kSteps; step += kAhead) {
+#pragma unroll
+                for (int half = 0; half < kAhead; ++half, it = next(it), ahead = next(ahead)) {
+                    if (kSteps % kAhead != 0 && step + half >= kSteps) break;
+                    const Fetched f = ring[half];
+                    if (step + half + kAhead < kSteps) fetch(ring[half], ahead, step + half + kAhead);
                     const bool here = valid(it);
                     if (!__any_sync(0xFFFFFFFFu, here)) continue;
                     const int yl = it.yl, arow = arow0 + yl, bsnp = tl.y * NZ + it.z;
@@ -809,8 +816,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                     if (wide) {
 #pragma unroll
                         for (int i = 0; i < NSEG / 2; ++i) {
-                            const float4 a = stash_counts<NZ>(slot, 1, i, etid + (step + half) * kScoreThreads);
-                            const float4 b = stash_counts<NZ>(slot, 1, NSEG / 2 + i, etid + (step + half) * kScoreThreads);
+                            const int idx = etid + (step + half) * kScoreThreads;
+                            const float4 a = stash_counts<NZ>(slot, 1, i, idx);
+                            const float4 b = nseg == NSEG ? stash_counts<NZ>(slot, 1, NSEG / 2 + i, idx) : make_float4(0, 0, 0, 0);
                             c[i][0][0] = pack2(a.x + off, b.x + off);
                             c[i][0][1] = pack2(a.y + off, b.y + off);
                             c[i][1][0] = pack2(a.z + off, b.z + off);

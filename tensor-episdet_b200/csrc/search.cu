@@ -165,9 +165,12 @@ cudaError_t timer_end(Workspace* w) {
 // Score tables, built on the host in double with glibc (src/search-pairs.cu:83-106):
 // K2 holds lnGamma(v+1) for v in [0, N+1]; MI holds log2(v * invN) for v in [1, N].
 episdet_status build_tables(Workspace* w, int score, int nc, int nn, ScoreTables* T) {
-    if (w->tab_score != score || w->tab_nc != nc || w->tab_nn != nn) {
-        int N = nc + nn;
-        int size = score == EPISDET_SCORE_K2 ? N + 2 : N + 1;
+    // The K2 table does not depend on the sample counts: a longer one serves.
+    const int N = nc + nn, size = score == EPISDET_SCORE_K2 ? N + 2 : N + 1;
+    const bool held = score == EPISDET_SCORE_K2 ? w->tab_score == score && w->tab_size >= size
+                                                : w->tab_score == score && w->tab_nc == nc && w->tab_nn == nn;
+    if (!held) {
+        w->tab_score = -1;
         std::vector<float> t32((size_t)size);
         std::vector<double> t64((size_t)size);
         if (score == EPISDET_SCORE_K2) {
@@ -200,6 +203,7 @@ episdet_status build_tables(Workspace* w, int score, int nc, int nn, ScoreTables
         CUDA_TRY(cudaStreamSynchronize(w->st));
         w->h2d += (int64_t)size * (sizeof(float) + sizeof(double));
         w->tab_score = score;
+        w->tab_size = size;
         w->tab_nc = nc;
         w->tab_nn = nn;
     }

@@ -90,7 +90,7 @@ struct Workspace {
     int64_t count_launches = 0;
     double executed_macs = 0.0;
     std::vector<double> launch_ms, launch_macs;  // EPISDET_FLAG_TIMING: per counting launch of the last call
-    int tab_score = -1, tab_nc = -1, tab_nn = -1;
+    int tab_score = -1, tab_size = 0, tab_nc = -1, tab_nn = -1;
     int stage_override = -1;  // triplet tiles: -1 by the panel-size rule, 0 narrow, 1 wide
     int pairs[16] = {};       // resident CTA pairs of each counting-kernel instance (0: not asked yet)
     float inv32 = 0.0f, hy32 = 0.0f;

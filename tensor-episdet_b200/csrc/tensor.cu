@@ -733,6 +733,7 @@ episdet_status tensor_pair_totals(Workspace* w, const uint32_t* d_planes, int M,
     p.ntiles = (int)tiles.size();
     p.seg2[0] = Seg{0, (n + kF4PerKB - 1) / kF4PerKB};
     p.wide = counts_wide(n, 0);
+    p.one_class = 1;
     p.out = (float*)out;
     p.out_n = 4;
     p.out_ld = M;
@@ -877,6 +878,7 @@ static episdet_status run_pairs(Workspace* w, const DevData& D, const episdet_op
     p.seg2[0] = Seg{0, (D.n[0] + kF4PerKB - 1) / kF4PerKB};
     p.seg2[1] = label ? Seg{kb1, kb1} : Seg{kb1, kb1 + (D.n[1] + kF4PerKB - 1) / kF4PerKB};
     p.tot = w->label_tot;
+    p.one_class = label;
     p.ngroup = 1;
     p.tiles = (const int2*)w->tiles.p;
     p.ntiles = (int)tiles.size();
