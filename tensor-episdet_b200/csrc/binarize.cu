@@ -7,144 +7,140 @@
 // genotype bytes and a case flag per sample.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 
+#include "common.cuh"
 #include "episdet.h"
 #include "host_util.h"
 #include "search_internal.h"
-#include "tc_ptx.cuh"
 
 namespace episdet {
 
 // Sample lists, cases then controls, each in sample order, and *num_cases.
-// One CTA: every thread counts, then lists, one stretch of samples.
+// One CTA: every warp counts, then lists, one stretch of samples, a lane each.
 constexpr int kListThreads = 1024;
 __global__ void __launch_bounds__(kListThreads) class_lists_kernel(const uint8_t* __restrict__ is_case, int n,
                                                                    int* __restrict__ idx, int* __restrict__ num_cases) {
     __shared__ int s_warp[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int per = (n + kListThreads - 1) / kListThreads;
-    const int s0 = min(n, (int)threadIdx.x * per), s1 = min(n, s0 + per);
+    const int per = (n + kListThreads - 1) / kListThreads * 32;  // samples of a warp
+    const int s0 = min(n, warp * per), s1 = min(n, s0 + per);
     int cnt = 0;
-    for (int i = s0; i < s1; ++i) cnt += __ldg(is_case + i) != 0;
-    int x = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) s_warp[warp] = x;
+#pragma unroll 8
+    for (int i = s0; i < s1; i += 32)
+        cnt += __popc(__ballot_sync(0xFFFFFFFFu, i + lane < s1 && __ldg(is_case + i + lane) != 0));
+    if (lane == 0) s_warp[warp] = cnt;
     __syncthreads();
     int below = 0, total = 0;
     for (int i = 0; i < 32; ++i) {
         below += i < warp ? s_warp[i] : 0;
         total += s_warp[i];
     }
-    int ic = below + x - cnt, in = total + s0 - ic;
-    for (int i = s0; i < s1; ++i) idx[__ldg(is_case + i) != 0 ? ic++ : in++] = i;
+    int ic = below, in = total + s0 - below;
+#pragma unroll 8
+    for (int i = s0; i < s1; i += 32) {
+        const bool here = i + lane < s1, is = here && __ldg(is_case + i + lane) != 0;
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, is), v = __ballot_sync(0xFFFFFFFFu, here);
+        const uint32_t lower = (1u << lane) - 1u;
+        if (here) idx[is ? ic + __popc(m & lower) : in + __popc(~m & lower)] = i + lane;
+        ic += __popc(m);
+        in += __popc(v & ~m);
+    }
     if (threadIdx.x == 0) *num_cases = total;
 }
 
-// One warp per kBinSnps SNPs x 32 output words of a class.  The 1,024 samples of
-// those words lie in one stretch of each genotype row: the warp copies the
-// stretch into shared memory (kBinSpan bytes at most; a class so sparse that it
-// is longer reads the row instead), and for each word the lanes read its 32
-// samples' bytes and two ballots make the plane words; lane k keeps word k, so
-// the stores are whole lines.  The bound is reading every genotype byte once
-// per class (8192 x 50001: 79 us for once at the copy rate); a thread per word,
-// each reading its own 32 samples, took 1700 us there, ballots over global
-// bytes 421 us, this BIN_US us.
+// The matrix is packed first, 16 SNPs of a sample to a word (bits 2 s and 2 s + 1:
+// genotype of SNP s is 0, 1), so that a class's samples are gathered a word at a
+// time and a 32 x 32 bit transpose of 32 samples gives the plane words of all 16
+// SNPs.  The bound is reading the bytes (79 us for 8192 x 50001 at the copy rate,
+// and a quarter of them written and read as words); a thread per output word,
+// each reading its own 32 samples, took 1700 us there, two ballots per SNP and
+// word 421 us.
 constexpr int kBinSnps = 16;
-constexpr int kBinSpan = 4096;
-constexpr int kBinWarps = 4;
+
+// Four samples of 16 SNPs a thread.
+__global__ void __launch_bounds__(256) pack_genotypes_kernel(const uint8_t* __restrict__ geno, int M, int n,
+                                                             uint32_t* __restrict__ packed, int pitch,
+                                                             int* __restrict__ bad) {
+    const int i0 = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x), snp0 = (int)blockIdx.y * kBinSnps;
+    if (i0 >= n) return;
+    const int ns = min(kBinSnps, M - snp0);
+    uint32_t acc[4] = {0, 0, 0, 0}, over = 0;
+    auto add = [&](int s, uint32_t x) {
+        over |= (x & 0xFCFCFCFCu) | (x & (x >> 1) & 0x01010101u);
+        const uint32_t code = (~(x | (x >> 1)) & 0x01010101u) | ((x & 0x01010101u) << 1);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[e] |= ((code >> (8 * e)) & 3u) << (2 * s);
+    };
+    // Four bytes at any alignment are two aligned words, where those lie in the
+    // matrix for all 16 rows; else one byte at a time (2 past the row's end).
+    const uint8_t* first = geno + (size_t)snp0 * n + i0;
+    if (ns == kBinSnps && i0 + 4 <= n && first - geno >= 3 &&
+        first + (size_t)(kBinSnps - 1) * n + 8 <= geno + (size_t)M * n) {
+        uint32_t lo[kBinSnps], hi[kBinSnps];
+#pragma unroll
+        for (int s = 0; s < kBinSnps; ++s) {
+            const uint8_t* p = first + (size_t)s * n;
+            const uint32_t* base = reinterpret_cast<const uint32_t*>(p - ((uintptr_t)p & 3));
+            lo[s] = __ldg(base);
+            hi[s] = __ldg(base + 1);
+        }
+#pragma unroll
+        for (int s = 0; s < kBinSnps; ++s)
+            add(s, __funnelshift_r(lo[s], hi[s], 8 * (int)((uintptr_t)(first + (size_t)s * n) & 3)));
+    } else {
+        for (int s = 0; s < ns; ++s) {
+            const uint8_t* p = first + (size_t)s * n;
+            uint32_t x = 0;
+            for (int e = 0; e < 4; ++e) x |= (uint32_t)(i0 + e < n ? p[e] : 2) << (8 * e);
+            add(s, x);
+        }
+    }
+    *reinterpret_cast<uint4*>(packed + (size_t)blockIdx.y * pitch + i0) = make_uint4(acc[0], acc[1], acc[2], acc[3]);
+    if (over) atomicExch(bad, 1);
+}
+
+// One warp per 16 SNPs x 8 output words of a class: lane l gathers the word's
+// sample l and, after the transpose, holds row l (SNP l / 2, plane l % 2); eight
+// words make its 32-byte store.
 struct BinClass {
     const int* idx;  // samples of the class
     uint32_t* out;   // [M][2][W]
     int n, W;
 };
-__global__ void __launch_bounds__(32 * kBinWarps) binarize_kernel(const uint8_t* __restrict__ geno, int M, int n,
-                                                                  BinClass a, BinClass b, int* __restrict__ bad) {
-    __shared__ __align__(16) uint8_t s_row[kBinWarps][2][kBinSpan + 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wa = a.W / 32, wb = b.W / 32;
-    const long unit = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // both classes of an SNP group together
-    const long group = unit / (wa + wb);
-    const int chunk = (int)(unit % (wa + wb));
-    if (group * kBinSnps >= M) return;
+__global__ void __launch_bounds__(256) planes_kernel(const uint32_t* __restrict__ packed, int pitch, int M, BinClass a,
+                                                     BinClass b) {
+    const int lane = threadIdx.x & 31, wa = a.W / 8, wb = b.W / 8;
+    const int chunk = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), snp0 = (int)blockIdx.y * kBinSnps;
+    if (chunk >= wa + wb) return;  // uniform over the warp
     const bool second = chunk >= wa;
     const int* __restrict__ idx = second ? b.idx : a.idx;
     uint32_t* __restrict__ out = second ? b.out : a.out;
     const int nk = second ? b.n : a.n, W = second ? b.W : a.W;
-    const int w0 = (second ? chunk - wa : chunk) * 32, i0 = w0 * 32;
-    const int snp0 = (int)group * kBinSnps, ns = min(kBinSnps, M - snp0);
-    // The stretch [lo, hi) of a row (empty when the words are all padding).
-    const int lo = i0 < nk ? __ldg(idx + i0) : 0, hi = i0 < nk ? __ldg(idx + min(nk, i0 + 1024) - 1) + 1 : 0;
-    const bool staged = hi - lo <= kBinSpan;
-    uint16_t rel[32];  // this lane's sample of each word, from lo
+    const int w0 = (second ? chunk - wa : chunk) * 8;
+    const uint32_t* __restrict__ p = packed + (size_t)blockIdx.y * pitch;
+    uint32_t v[8];
 #pragma unroll
-    for (int k = 0; k < 32; ++k) {
-        const int i = i0 + k * 32 + lane;
-        rel[k] = staged && i < nk ? (uint16_t)(__ldg(idx + i) - lo) : 0xFFFFu;
+    for (int k = 0; k < 8; ++k) {
+        const int i = (w0 + k) * 32 + lane;
+        v[k] = i < nk ? __ldg(p + __ldg(idx + i)) : 0u;
     }
-    // Copies a row's stretch: whole aligned 16 bytes, byte by byte where they
-    // would leave the row.  Returns where the stretch begins in the buffer.
-    auto copy = [&](int s) {
-        const uint8_t* g0 = geno + (size_t)(snp0 + s) * n;
-        const uint8_t* from = g0 + lo;
-        const int skew = (int)((uintptr_t)from & 15);
-        const uint8_t* base = from - skew;
-        uint8_t* row = s_row[warp][s & 1];
-        for (int o = 16 * lane; o < hi - lo + skew; o += 512) {
-            const uint8_t* p = base + o;
-            if (p >= g0 && p + 16 <= g0 + n) {
-                ptx::cp_async16(ptx::smem_u32(row + o), p, true);
-            } else {
-                for (int e = 0; e < 16; ++e)
-                    if (p + e >= from && p + e < g0 + hi) row[o + e] = p[e];
-            }
-        }
-        ptx::cp_async_commit();
-        return skew;
-    };
-    bool over = false;
-    int skew = 0, skew_next = staged ? copy(0) : 0;
-    for (int s = 0; s < ns; ++s) {
-        const uint8_t* g0 = geno + (size_t)(snp0 + s) * n;
-        uint32_t p0 = 0, p1 = 0;
-        skew = skew_next;
-        if (staged) {
-            // The next row's copy is in flight while this one is read.
-            if (s + 1 < ns) {
-                skew_next = copy(s + 1);
-                ptx::cp_async_wait<1>();
-            } else {
-                ptx::cp_async_wait<0>();
-            }
-            __syncwarp();
-            const uint8_t* row = s_row[warp][s & 1] + skew;
+    // warp_transpose32 gives lane l the words' bits 31 - l, first lane first.
 #pragma unroll
-            for (int k = 0; k < 32; ++k) {
-                const uint32_t g = rel[k] != 0xFFFFu ? row[rel[k]] : 2u;
-                const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, g == 0), m1 = __ballot_sync(0xFFFFFFFFu, g == 1);
-                over |= g > 2;
-                if (lane == k) p0 = m0, p1 = m1;
-            }
-            __syncwarp();  // before the buffer's next copy
-        } else {
-            for (int k = 0; k < 32; ++k) {
-                const int i = i0 + k * 32 + lane;
-                const uint32_t g = i < nk ? __ldg(g0 + __ldg(idx + i)) : 2u;
-                const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, g == 0), m1 = __ballot_sync(0xFFFFFFFFu, g == 1);
-                over |= g > 2;
-                if (lane == k) p0 = m0, p1 = m1;
-            }
+    for (int k = 0; k < 8; ++k) v[k] = warp_transpose32(v[k], lane);
+    const int bit = 31 - lane, snp = snp0 + bit / 2;
+    if (snp < M) {
+        uint32_t* o = out + ((size_t)snp * 2 + bit % 2) * W + w0;
+        if (((uintptr_t)o & 15) == 0) {
+            reinterpret_cast<uint4*>(o)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+            reinterpret_cast<uint4*>(o)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+        } else {  // the caller's array
+#pragma unroll
+            for (int k = 0; k < 8; ++k) o[k] = v[k];
         }
-        uint32_t* o = out + (size_t)(snp0 + s) * 2 * W + w0 + lane;
-        o[0] = __brev(p0);
-        o[W] = __brev(p1);
     }
-    if (__any_sync(0xFFFFFFFFu, over) && lane == 0) atomicExch(bad, 1);
 }
 
 }  // namespace episdet
@@ -200,10 +196,23 @@ extern "C" episdet_status episdet_binarize(const uint8_t* genotypes, int32_t num
             d_out[c] = (uint32_t*)w->bin_out[c].p;
         }
     }
+    const int groups = (M + kBinSnps - 1) / kBinSnps, pitch = (n + 3) & ~3;
     const BinClass ca{d_idx, d_out[0], nc, Wc}, cb{d_idx + nc, d_out[1], nn, Wn};
-    const long warps = (long)((M + kBinSnps - 1) / kBinSnps) * (Wc / 32 + Wn / 32);
-    binarize_kernel<<<(unsigned)((warps + kBinWarps - 1) / kBinWarps), 32 * kBinWarps, 0, s>>>(d_geno, M, n, ca, cb, d_flag);
-    CHECK_LAUNCH();
+    // SNP groups in batches of at most 512 MB of words (and of the grid's second dimension).
+    const int batch = (int)std::max<size_t>(1, std::min<size_t>(32768, ((size_t)512 << 20) / (sizeof(uint32_t) * (size_t)pitch)));
+    CUDA_TRY(w->bin_pack.ensure(sizeof(uint32_t) * (size_t)std::min(groups, batch) * pitch));
+    uint32_t* d_pack = (uint32_t*)w->bin_pack.p;
+    for (int g0 = 0; g0 < groups; g0 += batch) {
+        const int ng = std::min(batch, groups - g0), r0 = g0 * kBinSnps, rows = std::min(M - r0, ng * kBinSnps);
+        pack_genotypes_kernel<<<dim3((unsigned)((pitch / 4 + 255) / 256), (unsigned)ng), 256, 0, s>>>(
+            d_geno + (size_t)r0 * n, rows, n, d_pack, pitch, d_flag);
+        CHECK_LAUNCH();
+        BinClass ga = ca, gb = cb;
+        ga.out += (size_t)r0 * 2 * Wc;
+        gb.out += (size_t)r0 * 2 * Wn;
+        planes_kernel<<<dim3((unsigned)((Wc / 8 + Wn / 8 + 7) / 8), (unsigned)ng), 256, 0, s>>>(d_pack, pitch, rows, ga, gb);
+        CHECK_LAUNCH();
+    }
     int bad = 0;
     CUDA_TRY(cudaMemcpyAsync(&bad, w->flag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     if (memory == EPISDET_HOST) {

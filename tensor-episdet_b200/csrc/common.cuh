@@ -269,6 +269,24 @@ struct LocalTopK {
     }
 };
 
+// 32 x 32 bit transpose across a warp: lane k returns the word whose bit
+// 31 - l is bit 31 - k of lane l's word (the block-swap transpose of
+// H. S. Warren, Hacker's Delight, 2nd ed., section 7-3, one stage per
+// shuffle distance).
+__device__ __forceinline__ uint32_t warp_transpose32(uint32_t a, int lane) {
+    uint32_t m = 0x0000FFFFu;
+#pragma unroll
+    for (int j = 16; j != 0; j >>= 1, m ^= m << j) {
+        const uint32_t p = __shfl_xor_sync(0xFFFFFFFFu, a, j);
+        if (lane & j) {
+            a ^= ((p ^ (a >> j)) & m) << j;
+        } else {
+            a ^= (a ^ (p >> j)) & m;
+        }
+    }
+    return a;
+}
+
 struct BarAll {
     __device__ void operator()() const { __syncthreads(); }
     __device__ bool any(bool q) const { return __syncthreads_or(q) != 0; }

@@ -81,7 +81,7 @@ struct Workspace {
     DevBuf perm_tt, perm_marg, perm_labels, perm_mask;  // label mode: transposed planes, genotype counts, labels, class masks
     const float4* label_tot = nullptr;  // set during a label-mode 2-way search (episdet_search_perm)
     DevBuf perm_planes, perm_cls[2], perm_idx;  // phenotype-permutation staging
-    DevBuf bin_geno, bin_idx, bin_out[2];       // genotype-matrix binarizer staging
+    DevBuf bin_geno, bin_idx, bin_pack, bin_out[2];       // genotype-matrix binarizer staging
     // Per-call accounting.
     int64_t h2d = 0, d2h = 0;
     bool timing = false;
@@ -103,7 +103,7 @@ struct Workspace {
                          &counts, &tiles, &merged, &flag, &frows, &rtab, &stash, &seeds, &planes_t[0], &planes_t[1],
                          &xinfo,
                          &tensor_flag, &cbuf, &perm_tot, &perm_tt, &perm_marg, &perm_labels, &perm_mask, &perm_planes, &perm_cls[0], &perm_cls[1], &perm_idx,
-                         &bin_geno, &bin_idx, &bin_out[0], &bin_out[1]};
+                         &bin_geno, &bin_idx, &bin_pack, &bin_out[0], &bin_out[1]};
         for (DevBuf* b : all) b->release();
         results.release();
         tab_score = tab_nc = tab_nn = -1;

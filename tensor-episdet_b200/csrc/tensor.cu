@@ -320,24 +320,6 @@ struct CmpOut {
 // back into rows by a 32 x 32 bit transpose in registers (five shuffle
 // stages).
 
-// 32 x 32 bit transpose across a warp: lane k returns the word whose bit
-// 31 - l is bit 31 - k of lane l's word (the block-swap transpose of
-// H. S. Warren, Hacker's Delight, 2nd ed., section 7-3, one stage per
-// shuffle distance).
-__device__ __forceinline__ uint32_t warp_transpose32(uint32_t a, int lane) {
-    uint32_t m = 0x0000FFFFu;
-#pragma unroll
-    for (int j = 16; j != 0; j >>= 1, m ^= m << j) {
-        const uint32_t p = __shfl_xor_sync(0xFFFFFFFFu, a, j);
-        if (lane & j) {
-            a ^= ((p ^ (a >> j)) & m) << j;
-        } else {
-            a ^= (a ^ (p >> j)) & m;
-        }
-    }
-    return a;
-}
-
 // Rows padded to whole 256-row tiles in the sample-major layout.
 constexpr int kTtRows = 256;
 __host__ __device__ inline int tt_row_words(int rows) { return (rows + kTtRows - 1) / kTtRows * (kTtRows / 32); }
@@ -677,7 +659,7 @@ static int first_b(int a, int nz) { return (kTileA * a) / nz; }
 // reaches past the A tile's first SNP, in bands of about 1024 x 1008 SNPs: the 74
 // tiles that run at once then read 8 + 9 row panels instead of 1 + 74 (all pairs
 // of 16384 SNPs x 32768 samples, whose rows are 537 MB: row by row 5.98 ms,
-// in bands BAND_MS).
+// in bands 4.89).
 static void pair_tiles(int M, int a0, int a1, int nz, std::vector<int2>& out) {
     constexpr int kBandA = 8;
     const int band_b = 9 * kWideZ / nz, ntb = (M + nz - 1) / nz;
@@ -978,23 +960,27 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
         CUDA_TRY(w->rtab.ensure(sizeof(float2) * 9 * (size_t)p.rt_ld * gmax));
         st = prepare_stash(w, nz, 4, (int64_t)D.n[0] + D.n[1] > 131070 || counts_wide(D.n[0], D.n[1]), &p);
         if (st != EPISDET_OK) return st;
-        size_t fr = 0, tot = 0;
-        CUDA_TRY(cudaMemGetInfo(&fr, &tot));
-        // Left for the tile lists, slots, merge buffers and the driver.
-        const size_t reserve = std::max<size_t>(tot / 32, (size_t)1 << 30);
-        // The pair-table buffers are replaced when they grow, so their memory counts as free.
-        const size_t held = w->ptab.cap + w->ptabx.cap;
-        const size_t avail = fr + held > reserve ? fr + held - reserve : 0;
         if (o.pair_block_snps > 0) {
             blk_tiles = std::min(blk_tiles, (o.pair_block_snps + kTileA - 1) / kTileA);
-        } else if (row_bytes * (size_t)M > avail) {
-            const size_t left = avail > xrows_bytes ? avail - xrows_bytes : 0;
-            blk_tiles = (int)std::min<size_t>((size_t)blk_tiles, left / (row_bytes * kTileA));
-            if (blk_tiles < 1)
-                return set_error(EPISDET_ERR_OUT_OF_MEMORY,
-                                 "3-way search of %d SNPs: no 128-row block of the pair table fits in the %.1f GB "
-                                 "left beside the operand buffers",
-                                 M, (double)avail / 1e9);
+        } else if (w->ptab.cap < row_bytes * (size_t)M) {
+            // (Asked for only when the table has to grow: on some hosts the
+            // driver takes 9 ms to answer, more than a small search.)
+            size_t fr = 0, tot = 0;
+            CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+            // Left for the tile lists, slots, merge buffers and the driver.
+            const size_t reserve = std::max<size_t>(tot / 32, (size_t)1 << 30);
+            // The pair-table buffers are replaced when they grow, so their memory counts as free.
+            const size_t held = w->ptab.cap + w->ptabx.cap;
+            const size_t avail = fr + held > reserve ? fr + held - reserve : 0;
+            if (row_bytes * (size_t)M > avail) {
+                const size_t left = avail > xrows_bytes ? avail - xrows_bytes : 0;
+                blk_tiles = (int)std::min<size_t>((size_t)blk_tiles, left / (row_bytes * kTileA));
+                if (blk_tiles < 1)
+                    return set_error(EPISDET_ERR_OUT_OF_MEMORY,
+                                     "3-way search of %d SNPs: no 128-row block of the pair table fits in the %.1f GB "
+                                     "left beside the operand buffers",
+                                     M, (double)avail / 1e9);
+            }
         }
         const bool blocked = blk_tiles < nt2 - a_first;
         CUDA_TRY(w->ptab.ensure(row_bytes * (blocked ? (size_t)blk_tiles * kTileA : (size_t)M)));

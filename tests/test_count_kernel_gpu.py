@@ -114,3 +114,27 @@ def test_binarize_groups_and_chunks(episdet, oracle, M, n):
     flags[0], flags[-1] = True, False
     cases, controls, nc, nn = episdet.binarize(g, flags)
     assert np.array_equal(cases, oracle.pack(g[:, flags])) and np.array_equal(controls, oracle.pack(g[:, ~flags]))
+
+
+def test_binarize_unaligned_device_arrays(episdet, oracle):
+    """Device arrays that start at odd bytes (genotypes) and words (planes)."""
+    import numpy as np
+    import torch
+
+    M, n = 19, 1301
+    rng = np.random.default_rng(3)
+    g = rng.integers(0, 3, size=(M, n)).astype(np.uint8)
+    flags = (rng.random(n) < 0.5).astype(np.uint8)
+    nc = int(flags.sum())
+    wc, wn = episdet.class_words(nc), episdet.class_words(n - nc)
+    dg = torch.zeros(M * n + 1, dtype=torch.uint8, device="cuda")
+    dg[1:] = torch.from_numpy(g.reshape(-1)).cuda()
+    df = torch.from_numpy(flags).cuda()
+    out = [torch.zeros(M * 2 * w + 1, dtype=torch.int32, device="cuda") for w in (wc, wn)]
+    torch.cuda.synchronize()
+    st = episdet.lib().episdet_binarize(dg.data_ptr() + 1, M, n, df.data_ptr(), out[0].data_ptr() + 4,
+                                        out[1].data_ptr() + 4, episdet.DEVICE, 0)
+    assert st == 0
+    for o, cls in zip(out, (flags != 0, flags == 0)):
+        got = o.cpu().numpy().view(np.uint32)
+        assert got[0] == 0 and np.array_equal(got[1:], oracle.pack(g[:, cls]).reshape(-1))
