@@ -371,12 +371,22 @@ __device__ __noinline__ void reach_level(const Slots& S, const uint32_t* s_level
     int j = 0;
     while (j + 1 < kLevels && key <= s_level[j + 1]) ++j;
     atomicAdd(&S.level_count[j], 1);
+    // (All counts at once: one trip to L2.  Their order does not matter, since
+    // each only grows.)
+    int4 c[kLevels / 4];
+#pragma unroll
+    for (int i = 0; i < kLevels / 4; ++i) c[i] = __ldcg(reinterpret_cast<const int4*>(S.level_count) + i);
     int below = 0;
-    for (int i = kLevels - 1; i >= 0; --i) {
-        below += *(volatile int*)&S.level_count[i];
-        if (below >= S.k) {
-            atomicMin(S.gkey, s_level[i]);
-            return;
+#pragma unroll
+    for (int i = kLevels / 4 - 1; i >= 0; --i) {
+        const int v[4] = {c[i].x, c[i].y, c[i].z, c[i].w};
+#pragma unroll
+        for (int e = 3; e >= 0; --e) {
+            below += v[e];
+            if (below >= S.k) {
+                atomicMin(S.gkey, s_level[4 * i + e]);
+                return;
+            }
         }
     }
 }

@@ -284,6 +284,7 @@ episdet_status prepare_slots(Workspace* w, int nslots, int k, Slots* S) {
     // Thresholds, search-wide key (both worst: all ones), counts (zero).
     // Then the threshold levels and their counts (none: zero).
     const size_t ones = sizeof(Cand) * ((size_t)nslots + 1), zeros = sizeof(int) * ((size_t)nslots + 2 * kLevels);
+    static_assert(sizeof(Cand) == 16 && kLevels % 4 == 0, "level counts are read 16 bytes at a time");
     CUDA_TRY(w->counts.ensure(ones + zeros));
     CUDA_TRY(cudaMemsetAsync(w->counts.p, 0xFF, ones, w->st));
     CUDA_TRY(cudaMemsetAsync((char*)w->counts.p + ones, 0, zeros, w->st));
@@ -291,9 +292,9 @@ episdet_status prepare_slots(Workspace* w, int nslots, int k, Slots* S) {
     S->ld = k;
     S->thr = (Cand*)w->counts.p;
     S->gkey = (uint32_t*)((Cand*)w->counts.p + nslots);
-    S->counts = (int*)((char*)w->counts.p + ones);
-    S->level = (uint32_t*)(S->counts + nslots);
-    S->level_count = S->counts + nslots + kLevels;
+    S->level_count = (int*)((char*)w->counts.p + ones);
+    S->level = (uint32_t*)(S->level_count + kLevels);
+    S->counts = S->level_count + 2 * kLevels;
     S->nslots = nslots;
     S->k = k;
     return EPISDET_OK;

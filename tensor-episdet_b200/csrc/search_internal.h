@@ -54,7 +54,10 @@ constexpr int kXSets = 2;
 constexpr int kXGroup = 4;  // first SNPs per triplet launch at least
 constexpr int kGroupTiles = 16;                   // tiles per CTA pair that a triplet launch should have
 constexpr size_t kGroupBytes = (size_t)2 << 30;   // regrouped rows a launch may take for them
-constexpr int kNarrowTileSnps = 448;              // panels up to this size use narrow triplet tiles
+// Panels up to this size use narrow triplet tiles (the last wide tile of a row
+// is a large share of theirs): 256 SNPs x 4096 samples 0.73 ms narrow, 0.83
+// wide; 600 x 10007 3.01 and 3.11; 1536 x 40000 42.0 and 37.8.
+constexpr int kNarrowTileSnps = 704;
 
 struct Workspace {
     int device = 0;

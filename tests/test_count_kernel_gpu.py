@@ -1,6 +1,6 @@
 """The counting kernel at the edges of its tiles, against the oracle.
 
-Tiles are 128 A SNPs x 112 (wide) or 56 (narrow) B SNPs; panels of up to 448
+Tiles are 128 A SNPs x 112 (wide) or 56 (narrow) B SNPs; panels of up to 704
 SNPs run narrow triplet tiles, pairs run narrow tiles when wide ones are fewer
 than the CTA pairs.  Counts pass through a buffer of 16-bit values, or 32-bit
 ones for a first SNP with a kept genotype of more than 65,535 samples.  K is
@@ -32,12 +32,12 @@ def test_tile_edges(episdet, oracle, order, M, score):
 
 
 @pytest.mark.parametrize("score", ["k2", "mi"])
-@pytest.mark.parametrize("M,slab", [(448, (440, 0)), (449, (0, 1)), (449, (126, 129)), (672, (330, 336))])
+@pytest.mark.parametrize("M,slab", [(704, (696, 0)), (705, (0, 1)), (705, (126, 129)), (784, (330, 336))])
 def test_triplet_tile_widths_and_list_edges(episdet, oracle, M, slab, score):
     check(episdet, oracle, 3, M, 1300, 900, score, 1536, slab=slab)
 
 
-@pytest.mark.parametrize("order,M,slab", [(3, 24, (0, 0)), (3, 460, (3, 4)), (2, 40, (0, 0)), (2, 1500, (700, 703))])
+@pytest.mark.parametrize("order,M,slab", [(3, 24, (0, 0)), (3, 710, (3, 4)), (2, 40, (0, 0)), (2, 1500, (700, 703))])
 def test_counts_past_16_bits(episdet, oracle, order, M, slab):
     check(episdet, oracle, order, M, 170000, 150000, "k2", 64, maf=(0.3, 0.36), slab=slab,
           flags=(0, episdet.FLAG_FILTER_OFF))
