@@ -272,7 +272,7 @@ def batched_vs_plain(reps=2):
             "ratio": min(tp) / min(tb), "identical": same,
             "plain_rate": work / min(tp) / 1e12, "batched_rate": work / min(tb) / 1e12, "unit": UNIT,
             "batched_autotune": True,
-            "tuned_staged": sorted({(nc_ if nc_ < nn_ else nn_).bit_length() - 1: episdet.tuned_stage(3, "k2", nc_, nn_)
+            "tuned_wide": sorted({(nc_ if nc_ < nn_ else nn_).bit_length() - 1: episdet.tuned_stage(3, "k2", nc_, nn_)
                                     for _, _, nc_, nn_, _, o_ in co if o_ == 3}.items()),
             "timing": f"wall clock per pass, device-resident planes, best of {reps} after a warm-up pass"}
 
@@ -358,13 +358,12 @@ def ours(args):
 
             dist.destroy_process_group()
         return
-    # Roofline of the dominant kernel (the triplet tensor launches), this rank:
+    # Roofline of the dominant kernel (the triplet counting launches), this rank:
     # the e2m1 MACs it issues (2 ops each) per second of its launches, against
-    # the best rate measured for that instruction at the shape it issues
-    # (tcgen05.mma.cta_group::2.kind::mxf4, N = 112: four count segments of
-    # 112 accumulator columns plus the scale-factor columns fill the 512 TMEM
-    # columns; profiles/tcgen05_mma_peak.md), and beside it the N = 256 rate
-    # (the instruction's best at any shape) and the measured bf16 x 4 figure.
+    # the measured rate of its instruction at the shape it issues
+    # (tcgen05.mma.cta_group::2.kind::mxf4, N = 224, at the maximum SM clock;
+    # profiles/tcgen05_mma_peak.md), and beside it the N = 256 rate and the
+    # measured bf16 x 4 figure.
     peaks = {}
     pp = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(pp):
@@ -374,7 +373,7 @@ def ours(args):
     pk = os.path.join(ROOT, "profiles", "tcgen05_mma_peak.md")
     if os.path.exists(pk):
         for line in open(pk):
-            for key in ("mxf4_pair_n112_peak_tflops", "mxf4_pair_n256_peak_tflops"):
+            for key in ("mxf4_pair_n224_peak_tflops", "mxf4_pair_n256_peak_tflops"):
                 if line.startswith(key + ":"):
                     inst[key] = float(line.split(":")[1].split()[0])
     kern_ms = sum(r.count_kernel_ms for r, _ in res) / args.steps
@@ -384,13 +383,12 @@ def ours(args):
     exe_ops = 2.0 * r0.executed_macs
     algorithmic = alg_ops / (kern_ms * 1e-3) / 1e12
     executed = exe_ops / (kern_ms * 1e-3) / 1e12
-    peak = inst.get("mxf4_pair_n112_peak_tflops")
+    peak = inst.get("mxf4_pair_n224_peak_tflops")
     p256 = inst.get("mxf4_pair_n256_peak_tflops")
     roof = {"bound": "tensor", "achieved": executed, "peak": peak, "unit": "TFLOP/s",
             "frac": (executed / peak) if peak else None, "traffic": None,
-            "kernel": "episdet::tc::tc_kernel (triplets)",
-            "peak_source": "measured on this pool: kind::mxf4 CTA-pair MMA, M=256 N=112, 64 MMAs per commit "
-                           "(profiles/tcgen05_mma_peak.md)",
+            "kernel": "episdet::tc::count_kernel (triplets)",
+            "peak_source": "measured: kind::mxf4 CTA-pair MMA, M=256 N=224, at 1965 MHz (profiles/tcgen05_mma_peak.md)",
             "frac_of_n256_instruction_peak": (executed / p256) if p256 else None,
             "n256_instruction_peak_tflops": p256,
             "frac_of_4x_bf16_sustained": executed / (4.0 * bf16),
@@ -400,7 +398,7 @@ def ours(args):
             "note": "achieved = e2m1 MACs the kernel issues x 2 / its launch time; the engine regroups samples by "
                     "the first SNP's genotype (exact), so it issues 4.2x fewer MACs than the algorithmic 8 AND "
                     "cells x N per triplet counted in algorithmic_tflops"}
-    prof = os.path.join(ROOT, "profiles", "tc_kernel_triplets.md")
+    prof = os.path.join(ROOT, "profiles", "count_kernel_triplets.md")
     if os.path.exists(prof):
         for line in open(prof):
             if line.startswith("traffic_bytes_per_launch_scaled:"):

@@ -198,8 +198,8 @@ extern "C" episdet_status episdet_binarize(const uint8_t* genotypes, int32_t num
     }
     const int groups = (M + kBinSnps - 1) / kBinSnps, pitch = (n + 3) & ~3;
     const BinClass ca{d_idx, d_out[0], nc, Wc}, cb{d_idx + nc, d_out[1], nn, Wn};
-    // SNP groups in batches of at most 512 MB of words (and of the grid's second dimension).
-    const int batch = (int)std::max<size_t>(1, std::min<size_t>(32768, ((size_t)512 << 20) / (sizeof(uint32_t) * (size_t)pitch)));
+    // SNP groups in batches of at most 64 MB of words (and of the grid's second dimension).
+    const int batch = (int)std::max<size_t>(1, std::min<size_t>(32768, ((size_t)64 << 20) / (sizeof(uint32_t) * (size_t)pitch)));
     CUDA_TRY(w->bin_pack.ensure(sizeof(uint32_t) * (size_t)std::min(groups, batch) * pitch));
     uint32_t* d_pack = (uint32_t*)w->bin_pack.p;
     for (int g0 = 0; g0 < groups; g0 += batch) {

@@ -5,8 +5,8 @@
 // Replaces the host drivers src/search-pairs.cu:9-246 and
 // src/search-triplets.cu:8-305 of hiperbio/tensor-episdet.  Where those issue
 // ~700k launches and ~280k stream syncs for a 4096-SNP 3-way search, this
-// driver issues one persistent counting launch per first SNP (3-way) or one in
-// total (2-way), and synchronises once at the end.
+// driver issues one persistent counting launch per group of first SNPs (3-way) or
+// one in total (2-way), and synchronises for the input check and at the end.
 #include <algorithm>
 #include <atomic>
 #include <chrono>

@@ -52,7 +52,9 @@ struct HostBuf {
 // group g + kXSets - 1 (second stream) overlaps the counting launch of group g.
 constexpr int kXSets = 2;
 constexpr int kXGroup = 4;  // first SNPs per triplet launch at least
-constexpr int kGroupTiles = 16;                   // tiles per CTA pair that a triplet launch should have
+// Tiles per CTA pair that a triplet launch should have (1536 SNPs x 40000
+// samples: 8 39.8 ms, 16 39.0, 32 38.7 at twice the rows).
+constexpr int kGroupTiles = 16;
 constexpr size_t kGroupBytes = (size_t)2 << 30;   // regrouped rows a launch may take for them
 // Panels up to this size use narrow triplet tiles (the last wide tile of a row
 // is a large share of theirs): 256 SNPs x 4096 samples 0.73 ms narrow, 0.83

@@ -87,12 +87,6 @@ __device__ __forceinline__ void ld_stream8(const float* p, float4& a, float4& b)
                  : "l"(p));
 }
 
-// Prefetch of one TMA box into L2 (no shared memory, no completion).
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
-    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y)
-                 : "memory");
-}
-
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
@@ -260,16 +254,7 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 }
 // Pair MMA, issued by the even CTA: A rows 0..127 from CTA 0's and 128..255
 // from CTA 1's shared memory (same offsets), B rows likewise split by N.
-__device__ __forceinline__ void mma_u8_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// Pair MMA of packed e2m1 operands with block scales read from TMEM at sfa /
+// Packed e2m1 operands with block scales read from TMEM at sfa /
 // sfb (kind::mxf4, 32-value blocks), FP32 accumulate; K = 64 values per MMA.
 __device__ __forceinline__ void mma_mxf4_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                               uint32_t sfa, uint32_t sfb, uint32_t accumulate) {

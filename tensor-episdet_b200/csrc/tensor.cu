@@ -824,7 +824,8 @@ static episdet_status run_pairs(Workspace* w, const DevData& D, const episdet_op
     const int M = D.M, Kc = D.W[0] * 32, Kn = D.W[1] * 32;
     const bool label = w->label_tot != nullptr;
     const int a0 = fb / kTileA, a1 = (fe - 1) / kTileA + 1;
-    // Narrow tiles when wide ones would leave CTA pairs without work.
+    // Narrow tiles when wide ones would leave CTA pairs without work (512 SNPs:
+    // counting launch 33 us narrow, 48 us wide; 1000 SNPs 33 and 37).
     std::vector<int2> tiles;
     pair_tiles(M, a0, a1, kWideZ, tiles);
     const bool narrow = (int)tiles.size() < w->sms / 2;
@@ -944,7 +945,7 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
     // First SNPs of a launch: as many as give every CTA pair kGroupTiles tiles,
     // at least kXGroup, with at most kGroupBytes of regrouped rows (or kXGroup's).
     const size_t member_bytes = (size_t)rows * pitch;
-    const int gmax = (int)std::min<size_t>(kMaxGroup, std::max<size_t>(kXGroup, kGroupBytes / member_bytes));
+    int gmax = (int)std::min<size_t>(kMaxGroup, std::max<size_t>(kXGroup, kGroupBytes / member_bytes));
     int blk_tiles = nt2 - a_first;  // A pair tiles (128 Y SNPs) per Y block
     {
         const size_t row_bytes = 8 * sizeof(float) * (size_t)M;  // one table row, both classes
@@ -952,7 +953,18 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
         // The other buffers of the search first (their later ensure calls
         // find them in place); the pair table gets what is left.
         CUDA_TRY(w->frows.ensure((size_t)rows * pitch));
-        for (DevBuf& d : w->xsub) CUDA_TRY(d.ensure(member_bytes * gmax));
+        for (DevBuf& d : w->xsub) {
+            cudaError_t e = d.ensure(member_bytes * gmax);
+            if (e == cudaErrorMemoryAllocation && gmax > kXGroup) {
+                // Little memory left: the smallest launches.
+                cudaGetLastError();
+                gmax = kXGroup;
+                for (DevBuf& x : w->xsub) x.release();
+                for (DevBuf& x : w->xsub) CUDA_TRY(x.ensure(member_bytes * gmax));
+                break;
+            }
+            CUDA_TRY(e);
+        }
         for (int c = 0; c < 2; ++c)
             CUDA_TRY(w->planes_t[c].ensure(sizeof(uint32_t) * (size_t)D.W[c] * 32 * tt_row_words(rows)));
         CUDA_TRY(w->xinfo.ensure((size_t)kXSets * gmax * xstride));
