@@ -61,6 +61,7 @@ __host__ __device__ inline uint64_t set_key2(uint32_t a, uint32_t b) { return ((
 struct ScoreTables {
     const float* t32;   // K2: lnGamma(v+1); MI: log2(v/N), index 0 -> 0
     const double* t64;
+    int last;           // last index of both: N + 1 (K2), N (MI)
     float inv_n32;
     float hy32;
     double inv_n64;
@@ -68,15 +69,25 @@ struct ScoreTables {
     int score;          // 0 = K2, 1 = MI
 };
 
+// Table lookups.  Planes that break the input contract unchecked
+// (EPISDET_FLAG_NO_VALIDATE) give counts outside 0 .. N, whose lookups read the
+// table's last entry.
 struct LutGlobal {
     const float* __restrict__ t;
-    __device__ __forceinline__ float operator()(int v) const { return __ldg(t + v); }
+    uint32_t last;
+    __device__ __forceinline__ float operator()(int v) const { return __ldg(t + min((uint32_t)v, last)); }
+};
+struct Lut64 {
+    const double* __restrict__ t;
+    uint32_t last;
+    __device__ __forceinline__ double operator()(int v) const { return t[min((uint32_t)v, last)]; }
 };
 // FP32 score of one table, scoring.hpp:5-16 (K2 cell term t[ctrl] + t[case] -
 // t[ctrl+case+1]; MI terms), cells in index order.  SC: the score when fixed
 // at compile time (EPISDET_SCORE_K2 / _MI), -1 to read T.score.
-template <int NC, class Lut, int SC = -1>
-__device__ __forceinline__ float score32_lut(const ScoreTables& T, const Lut& lut, const int* cs, const int* cn) {
+template <int NC, int SC = -1>
+__device__ __forceinline__ float score32(const ScoreTables& T, const int* cs, const int* cn) {
+    const LutGlobal lut{T.t32, (uint32_t)T.last};
     if (SC == 0 || (SC < 0 && T.score == 0)) {
         float s = 0.0f;
 #pragma unroll
@@ -97,17 +108,13 @@ __device__ __forceinline__ float score32_lut(const ScoreTables& T, const Lut& lu
 }
 
 template <int NC>
-__device__ __forceinline__ float score32(const ScoreTables& T, const int* cs, const int* cn) {
-    return score32_lut<NC>(T, LutGlobal{T.t32}, cs, cn);
-}
-
-template <int NC>
 __device__ __forceinline__ double score64(const ScoreTables& T, const int* cs, const int* cn) {
+    const Lut64 lut{T.t64, (uint32_t)T.last};
     if (T.score == 0) {
         double s = 0.0;
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            double term = __dsub_rn(__dadd_rn(T.t64[cn[c]], T.t64[cs[c]]), T.t64[cn[c] + cs[c] + 1]);
+            double term = __dsub_rn(__dadd_rn(lut(cn[c]), lut(cs[c])), lut(cn[c] + cs[c] + 1));
             s = __dadd_rn(s, term);
         }
         return fabs(s);
@@ -116,10 +123,10 @@ __device__ __forceinline__ double score64(const ScoreTables& T, const int* cs, c
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
         double pc = __dmul_rn((double)cs[c], T.inv_n64);
-        ha = __fma_rn(-pc, T.t64[cs[c]], ha);
+        ha = __fma_rn(-pc, lut(cs[c]), ha);
         double pn = __dmul_rn((double)cn[c], T.inv_n64);
-        ha = __fma_rn(-pn, T.t64[cn[c]], ha);
-        hx = __fma_rn(-__dadd_rn(pc, pn), T.t64[cs[c] + cn[c]], hx);
+        ha = __fma_rn(-pn, lut(cn[c]), ha);
+        hx = __fma_rn(-__dadd_rn(pc, pn), lut(cs[c] + cn[c]), hx);
     }
     return __dsub_rn(__dadd_rn(hx, T.hy64), ha);
 }

@@ -112,7 +112,6 @@ struct CountParams {
     const float2* rt;
     int rt_ld;
     float tab_off;
-    int tab_last;       // last index of the score table
     PairView yv;        // triplets: pairs of the second and third SNP
     const float4* tot;  // label mode: [M][M] AND cells over all samples; controls = these - cases
     float* out;         // store mode: pair (r, col) at out + out_n * ((r - out_r0) * out_ld + col - out_c0)
@@ -309,13 +308,6 @@ __device__ __forceinline__ float4 stash_counts(const uint4* slot, int wide, int 
 // ------------------------------------------------------------ exact score
 // FP32 score of one set from its exact counts, in the reference's cell order.
 // Rare (the bound rules out nearly every set): everything is read again.
-// Planes that break the input contract unchecked (EPISDET_FLAG_NO_VALIDATE)
-// give impossible counts; they read the table's last entry.
-struct LutClamped {
-    const float* __restrict__ t;
-    uint32_t last;
-    __device__ __forceinline__ float operator()(int v) const { return __ldg(t + min((uint32_t)v, last)); }
-};
 template <int MODE, int SC, int NZ>
 __device__ __noinline__ float exact_score(const CountParams& P, const uint4* slot, int wide, int ga, int gb, int g,
                                           int idx, int arow, int bsnp) {
@@ -364,7 +356,7 @@ __device__ __noinline__ float exact_score(const CountParams& P, const uint4* slo
             t[8] = at(2, bsnp) - (t[2] + t[5]);
         }
     }
-    return score32_lut<NC, LutClamped, SC>(P.T, LutClamped{P.T.t32, (uint32_t)P.tab_last}, tab[0], tab[1]);
+    return score32<NC, SC>(P.T, tab[0], tab[1]);
 }
 
 // Counts a scored set of this key at the lowest level it reaches, and lowers

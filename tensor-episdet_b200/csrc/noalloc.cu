@@ -204,6 +204,7 @@ static episdet_status search_locked(const episdet_dataset* data, const episdet_o
         T.hy32 = mi_hy32(nc, nn, T.inv_n32, h_t32);
     }
     T.score = o.score;
+    T.last = size - 1;
     T.t32 = (const float*)(S + kOffT32);
     T.t64 = (const double*)(S + kOffT64);
     CUDA_TRY(cudaMemcpyAsync(S + kOffT32, h_t32, sizeof(float) * size, cudaMemcpyHostToDevice, stream));

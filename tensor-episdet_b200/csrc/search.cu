@@ -209,6 +209,7 @@ episdet_status build_tables(Workspace* w, int score, int nc, int nn, ScoreTables
     }
     T->t32 = (const float*)w->t32.p;
     T->t64 = (const double*)w->t64.p;
+    T->last = size - 1;
     T->inv_n32 = w->inv32;
     T->inv_n64 = w->inv64;
     T->hy32 = w->hy32;

@@ -911,7 +911,6 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
     // past that are scored exactly throughout.
     p.filter = (o.flags & EPISDET_FLAG_FILTER_OFF) == 0 && std::max(D.n[0], D.n[1]) <= (1 << 22);
     p.tab_off = p.filter && T.score == EPISDET_SCORE_K2 ? 3.0f * kCellOff<0> : 0.0f;
-    p.tab_last = D.n[0] + D.n[1] + (T.score == EPISDET_SCORE_K2 ? 1 : 0);
     bound_coefficients(T, D.n[0], D.n[1], o.order == 2 ? 9 : 27, &p);
 
     if (o.order == 2) return run_pairs(w, D, o, fb, fe, p, launches, progress);
