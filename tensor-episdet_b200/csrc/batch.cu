@@ -256,18 +256,19 @@ extern "C" episdet_status episdet_search_perm(const episdet_cohort* cohort, cons
     const uint32_t* d_labels = labels;
     std::vector<uint32_t> h_labels;
     if (label_mode) {
+        // On the call's stream: device labels may still be on their way there.
+        begin_call(w0, o);
         // The labels on both sides: the host counts their cases.
         const size_t words = (size_t)num_labels * W;
         if (on_device) {
             h_labels.resize(words);
-            CUDA_TRY(cudaMemcpyAsync(h_labels.data(), labels, sizeof(uint32_t) * words, cudaMemcpyDeviceToHost, w0->own_st));
+            CUDA_TRY(cudaMemcpyAsync(h_labels.data(), labels, sizeof(uint32_t) * words, cudaMemcpyDeviceToHost, w0->st));
         } else {
             CUDA_TRY(w0->perm_labels.ensure(sizeof(uint32_t) * words));
-            CUDA_TRY(cudaMemcpyAsync(w0->perm_labels.p, labels, sizeof(uint32_t) * words, cudaMemcpyHostToDevice, w0->own_st));
+            CUDA_TRY(cudaMemcpyAsync(w0->perm_labels.p, labels, sizeof(uint32_t) * words, cudaMemcpyHostToDevice, w0->st));
             d_labels = (const uint32_t*)w0->perm_labels.p;
         }
-        CUDA_TRY(cudaStreamSynchronize(w0->own_st));
-        begin_call(w0, o);
+        CUDA_TRY(cudaStreamSynchronize(w0->st));
         st = tensor_label_cohort(w0, &lc, !(o.flags & EPISDET_FLAG_NO_VALIDATE));
         if (st != EPISDET_OK) return with_prefix(st, "label", 0);
     }

@@ -397,6 +397,8 @@ static episdet_status finish(Workspace* w, const DevData& D, const ScoreTables& 
     const int cnt = ((const int*)w->results.p)[0], dev_err = ((const int*)w->results.p)[1];
     const Cand* cands = (const Cand*)((const char*)w->results.p + head);
     const double* f64 = (const double*)(cands + k);
+    if (dev_err == kErrLabelChanged)
+        return set_error(EPISDET_ERR_INVALID_ARGUMENT, "the label changed while the call was using it");
     if (dev_err)
         return set_error(EPISDET_ERR_TIMEOUT, "a bounded device wait gave up (code %d); results discarded", dev_err);
     if (cnt < 1) return set_error(EPISDET_ERR_INTERNAL, "no candidate survived the search");

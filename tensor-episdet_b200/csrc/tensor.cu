@@ -239,9 +239,12 @@ __global__ void __launch_bounds__(256) cohort_marginals_kernel(const uint32_t* _
 }
 
 // One label: the ascending case samples (as member 0's first segment of class
-// 0, the form the regrouping reads) and the two classes' masks.
+// 0, the form the regrouping reads) and the two classes' masks.  The operand
+// rows are sized for the nc cases that the host counted: a label whose words
+// have changed since is an error, and no more than nc samples are regrouped.
 __global__ void __launch_bounds__(kXinfoThreads) label_lists_kernel(const uint32_t* __restrict__ label, int n, int W,
-                                                                    XWork xw, uint32_t* __restrict__ mask) {
+                                                                    int nc, XWork xw, uint32_t* __restrict__ mask,
+                                                                    int* __restrict__ err) {
     __shared__ int s_warp[32];
     __shared__ int s_total;
     const int per = (W + kXinfoThreads - 1) / kXinfoThreads;
@@ -267,7 +270,8 @@ __global__ void __launch_bounds__(kXinfoThreads) label_lists_kernel(const uint32
     }
     if (threadIdx.x == 0) {
         XInfo* info = xw.info(0);
-        info->len[0][0] = s_total;
+        info->len[0][0] = min(s_total, nc);
+        if (s_total != nc) record_error(err, kErrLabelChanged);
         info->len[0][1] = info->len[1][0] = info->len[1][1] = 0;
     }
 }
@@ -791,7 +795,7 @@ episdet_status tensor_label_rows(Workspace* w, const LabelCohort& c, const uint3
     xw.x0 = 0;
     CUDA_TRY(w->xinfo.ensure(xw.stride));
     xw.base = (uint8_t*)w->xinfo.p;
-    label_lists_kernel<<<1, kXinfoThreads, 0, w->st>>>(d_label, c.n, c.W, xw, mask);
+    label_lists_kernel<<<1, kXinfoThreads, 0, w->st>>>(d_label, c.n, c.W, nc, xw, mask, (int*)w->tensor_flag.p);
     CHECK_LAUNCH();
     label_marginals_kernel<<<(c.M + 7) / 8, 256, 0, w->st>>>(c.planes, c.M, c.W, mask, nc, c.marg, (int*)w->marg[0].p,
                                                              (int*)w->marg[1].p);

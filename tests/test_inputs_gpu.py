@@ -2,9 +2,11 @@
 
 Planes that break the input contract under FLAG_NO_VALIDATE give counts outside
 0 .. N and scores that mean nothing; the call must still stay inside its tables
-and buffers and leave the next search correct.
+and buffers and leave the next search correct.  Device inputs may still be on
+their way on the stream that the call is given.
 """
-import numpy as np
+import ctypes
+
 import pytest
 
 from test_parity_gpu import assert_same
@@ -27,3 +29,33 @@ def test_impossible_counts_stay_inside_the_score_tables(episdet, oracle, engine,
         assert e.name == "EPISDET_ERR_INTERNAL"
     o = oracle.search(*good, nc, nn, order=order, score=score, top_k=k)
     assert_same(episdet.search(*good, nc, nn, order=order, score=score, top_k=k, engine=engine), o, k)
+
+
+def test_device_labels_still_being_written_on_the_callers_stream(episdet, oracle):
+    """The labels (all zero until then) arrive on the caller's stream behind a
+    wait of some tenths of a second, and are not what the buffer held before."""
+    import torch
+
+    n, M, nc, nl, k = 3000, 90, 1100, 3, 32
+    planes = episdet.generate_cohort(91, M, n)
+    labels = episdet.generate_labels(92, n, nc, nl)
+    dev = torch.from_numpy(planes.view("int32")).cuda()
+    new = torch.from_numpy(labels.view("int32")).cuda()
+    late = torch.zeros_like(new)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    c = episdet.Cohort(dev.data_ptr(), M, n, episdet.DEVICE)
+    o = episdet.make_options(2, "k2", k, stream=stream.cuda_stream)
+    rs, keep = (episdet.Result * nl)(), []
+    for i in range(nl):
+        rs[i], bufs = episdet._result_buffers(k)
+        keep.append(bufs)
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(400_000_000)
+        late.copy_(new)
+    assert not stream.query()  # the labels are not there yet
+    episdet._check(episdet.lib().episdet_search_perm(ctypes.byref(c), late.data_ptr(), nl, ctypes.byref(o), rs))
+    for i, lab in enumerate(labels):
+        a, b, na, nb = oracle.split_by_label(planes, n, lab)
+        want = oracle.search(a, b, na, nb, order=2, score="k2", top_k=k)
+        assert_same(episdet._to_result(2, rs[i], keep[i]), want, k)
