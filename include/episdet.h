@@ -104,7 +104,9 @@ typedef struct episdet_dataset {
     int32_t memory;           /* EPISDET_HOST or EPISDET_DEVICE (current device) */
 } episdet_dataset;
 
-/* One cohort without a class split (all samples as one plane set). */
+/* One cohort without a class split (all samples as one plane set).  Only the
+ * num_samples samples are read: padding bits of the planes and labels may hold
+ * anything. */
 typedef struct episdet_cohort {
     const uint32_t* planes;   /* [num_snps][2][episdet_class_words(num_samples)] */
     int32_t num_snps;

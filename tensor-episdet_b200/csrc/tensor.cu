@@ -46,7 +46,9 @@ __device__ __forceinline__ uint4 e2m1_word(uint32_t w) {
 // Packed planes -> packed e2m1 operand rows, in the class-region layout of the
 // regrouped triplet rows (no regrouping): row r = 2*snp + g holds the cases
 // from packed sample 0 and the controls from packed sample Kc + kClassPad.
-// One thread per source word.
+// Bits past a class's samples are left out (a cohort's may be set: its pair
+// totals count the samples that the labels split, no more).  One thread per
+// source word.
 __global__ void __launch_bounds__(256) pack_f4_kernel(DevData D, uint8_t* __restrict__ out, int rows, int pitch) {
     const int W0 = D.W[0], W1 = D.W[1], wpr = W0 + W1;
     const int base1 = (W0 * 32 + kClassPad) / 2;  // byte offset of the controls' region
@@ -55,7 +57,9 @@ __global__ void __launch_bounds__(256) pack_f4_kernel(DevData D, uint8_t* __rest
         const int r = (int)(t / wpr), w = (int)(t % wpr);
         const int c = w < W0 ? 0 : 1;
         const int ww = w - (c ? W0 : 0);
-        const uint32_t word = __ldg(D.bits[c] + (size_t)r * D.W[c] + ww);
+        const int left = D.n[c] - 32 * ww;  // samples from this word on
+        const uint32_t valid = left >= 32 ? ~0u : left > 0 ? ~0u << (32 - left) : 0u;
+        const uint32_t word = __ldg(D.bits[c] + (size_t)r * D.W[c] + ww) & valid;
         *reinterpret_cast<uint4*>(out + (size_t)r * pitch + (c ? base1 : 0) + (size_t)ww * 16) = e2m1_word(word);
     }
 }

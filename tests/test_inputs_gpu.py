@@ -3,10 +3,12 @@
 Planes that break the input contract under FLAG_NO_VALIDATE give counts outside
 0 .. N and scores that mean nothing; the call must still stay inside its tables
 and buffers and leave the next search correct.  Device inputs may still be on
-their way on the stream that the call is given.
+their way on the stream that the call is given, and a cohort's padding bits are
+not read.
 """
 import ctypes
 
+import numpy as np
 import pytest
 
 from test_parity_gpu import assert_same
@@ -29,6 +31,27 @@ def test_impossible_counts_stay_inside_the_score_tables(episdet, oracle, engine,
         assert e.name == "EPISDET_ERR_INTERNAL"
     o = oracle.search(*good, nc, nn, order=order, score=score, top_k=k)
     assert_same(episdet.search(*good, nc, nn, order=order, score=score, top_k=k, engine=engine), o, k)
+
+
+@pytest.mark.parametrize("score", ["k2", "mi"])
+def test_cohort_padding_bits_are_not_counted(episdet, oracle, score):
+    """Set bits past the last sample, of the planes and of the labels: label mode
+    and the per-label split give the answer of the clean cohort."""
+    n, M, nc, k = 2085, 60, 900, 50
+    planes = episdet.generate_cohort(17, M, n)
+    labels = episdet.generate_labels(18, n, nc, 2)
+    want = []
+    for lab in labels:
+        a, b, na, nb = oracle.split_by_label(planes, n, lab)
+        want.append(oracle.search(a, b, na, nb, order=2, score=score, top_k=k))
+    rng = np.random.default_rng(19)
+    for words in (planes, labels):
+        w = n // 32
+        words[..., w] |= rng.integers(0, 1 << (32 - n % 32), words[..., w].shape, dtype=np.uint32)
+        words[..., w + 1:] = rng.integers(0, 1 << 32, words[..., w + 1:].shape, dtype=np.uint32)
+    for flags in (0, episdet.FLAG_PERM_SPLIT):
+        for r, o in zip(episdet.search_perm(planes, n, labels, order=2, score=score, top_k=k, flags=flags), want):
+            assert_same(r, o, k)
 
 
 def test_device_labels_still_being_written_on_the_callers_stream(episdet, oracle):
