@@ -43,6 +43,7 @@ constexpr int kLevels = 16;
 // Codes of the tensor engine's error word; 1 to 7 are waits that gave up and
 // refused launches (count_kernel.cuh).
 constexpr int kErrLabelChanged = 8;  // a label is not the one its cases were counted from
+constexpr int kErrPlanes = 9;        // overlapping planes: a first SNP keeps more samples than its rows hold
 
 __device__ __forceinline__ void load_marg3(const int* m, int M, int snp, int out[3]) {
     out[0] = __ldg(m + snp);

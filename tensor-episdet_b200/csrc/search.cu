@@ -399,6 +399,8 @@ static episdet_status finish(Workspace* w, const DevData& D, const ScoreTables& 
     const double* f64 = (const double*)(cands + k);
     if (dev_err == kErrLabelChanged)
         return set_error(EPISDET_ERR_INVALID_ARGUMENT, "the label changed while the call was using it");
+    if (dev_err == kErrPlanes)
+        return set_error(EPISDET_ERR_INVALID_INPUT, "input planes have overlapping genotype-0/1 planes");
     if (dev_err)
         return set_error(EPISDET_ERR_TIMEOUT, "a bounded device wait gave up (code %d); results discarded", dev_err);
     if (cnt < 1) return set_error(EPISDET_ERR_INTERNAL, "no candidate survived the search");

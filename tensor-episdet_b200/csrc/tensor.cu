@@ -144,6 +144,7 @@ struct XWork {
     size_t info_bytes;
     int x0;
     int max_n;
+    int* err;
     __device__ __forceinline__ XInfo* info(int m) const { return reinterpret_cast<XInfo*>(base + m * stride); }
     __device__ __forceinline__ int* idx(int m) const { return reinterpret_cast<int*>(base + m * stride + info_bytes); }
 };
@@ -174,6 +175,7 @@ __global__ void __launch_bounds__(kXinfoThreads) xinfo_kernel(DevData D, XWork x
     const int w0 = threadIdx.x * per, w1 = min(W, w0 + per);
     // Class 1's region starts after class 0's Kc + kClassPad packed samples.
     const int base_kb = c == 0 ? 0 : (D.W[0] * 32 + kClassPad) / kF4PerKB;
+    const int end_kb = base_kb + (W * 32 + kClassPad) / kF4PerKB;
     int kb = base_kb;
     for (int s = 0; s < 2; ++s) {
         const int g = s == 0 ? ga : gb;
@@ -198,6 +200,11 @@ __global__ void __launch_bounds__(kXinfoThreads) xinfo_kernel(DevData D, XWork x
             }
         }
         int len = s_total;
+        // The two kept genotypes of disjoint planes fit the class's region.
+        if (kb + (len + kF4PerKB - 1) / kF4PerKB > end_kb) {
+            len = 0;
+            if (threadIdx.x == 0) record_error(xw.err, kErrPlanes);
+        }
         if (threadIdx.x == 0) {
             info->len[c][s] = len;
             info->seg[c * 2 + s].kb0 = kb;
@@ -247,8 +254,7 @@ __global__ void __launch_bounds__(256) cohort_marginals_kernel(const uint32_t* _
 // rows are sized for the nc cases that the host counted: a label whose words
 // have changed since is an error, and no more than nc samples are regrouped.
 __global__ void __launch_bounds__(kXinfoThreads) label_lists_kernel(const uint32_t* __restrict__ label, int n, int W,
-                                                                    int nc, XWork xw, uint32_t* __restrict__ mask,
-                                                                    int* __restrict__ err) {
+                                                                    int nc, XWork xw, uint32_t* __restrict__ mask) {
     __shared__ int s_warp[32];
     __shared__ int s_total;
     const int per = (W + kXinfoThreads - 1) / kXinfoThreads;
@@ -275,7 +281,7 @@ __global__ void __launch_bounds__(kXinfoThreads) label_lists_kernel(const uint32
     if (threadIdx.x == 0) {
         XInfo* info = xw.info(0);
         info->len[0][0] = min(s_total, nc);
-        if (s_total != nc) record_error(err, kErrLabelChanged);
+        if (s_total != nc) record_error(xw.err, kErrLabelChanged);
         info->len[0][1] = info->len[1][0] = info->len[1][1] = 0;
     }
 }
@@ -797,9 +803,10 @@ episdet_status tensor_label_rows(Workspace* w, const LabelCohort& c, const uint3
     xw.stride = (xw.info_bytes + sizeof(int) * 4 * (size_t)c.n + 255) & ~size_t(255);
     xw.max_n = c.n;
     xw.x0 = 0;
+    xw.err = (int*)w->tensor_flag.p;
     CUDA_TRY(w->xinfo.ensure(xw.stride));
     xw.base = (uint8_t*)w->xinfo.p;
-    label_lists_kernel<<<1, kXinfoThreads, 0, w->st>>>(d_label, c.n, c.W, nc, xw, mask, (int*)w->tensor_flag.p);
+    label_lists_kernel<<<1, kXinfoThreads, 0, w->st>>>(d_label, c.n, c.W, nc, xw, mask);
     CHECK_LAUNCH();
     label_marginals_kernel<<<(c.M + 7) / 8, 256, 0, w->st>>>(c.planes, c.M, c.W, mask, nc, c.marg, (int*)w->marg[0].p,
                                                              (int*)w->marg[1].p);
@@ -1104,6 +1111,7 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
         xw[b].stride = xstride;
         xw[b].info_bytes = info_bytes;
         xw[b].max_n = max_n;
+        xw[b].err = d_err;
         st = make_tmap(&tmx[b][0], w->xsub[b].p, (uint64_t)rows * gmax, (uint64_t)pitch, kCtaRows);
         if (st == EPISDET_OK) st = make_tmap(&tmx[b][1], w->xsub[b].p, (uint64_t)rows * gmax, (uint64_t)pitch, nz);
         if (st != EPISDET_OK) return st;

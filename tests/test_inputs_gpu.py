@@ -33,6 +33,24 @@ def test_impossible_counts_stay_inside_the_score_tables(episdet, oracle, engine,
     assert_same(episdet.search(*good, nc, nn, order=order, score=score, top_k=k, engine=engine), o, k)
 
 
+@pytest.mark.parametrize("full", [0, 1], ids=["cases", "controls"])
+def test_kept_samples_stay_inside_the_regrouped_rows(episdet, oracle, full):
+    """Both planes full in one class, genotype 2 the most frequent over both: the
+    two kept genotypes list that class's samples twice, more than a row holds."""
+    M, k = 150, 64
+    n = [3000, 3000]
+    n[full] = 1024  # 4 blocks of 256 samples a genotype; the class's region has 6
+    good = episdet.generate(0x1A8, M, *n)
+    bad = [p.copy() for p in good]
+    for c, p in enumerate(bad):
+        p[:, :, : n[c] // 32] = 0xFFFFFFFF if c == full else 0
+    with pytest.raises(episdet.EpisdetError) as e:
+        episdet.search(*bad, *n, order=3, top_k=k, engine="tensor", flags=episdet.FLAG_NO_VALIDATE)
+    assert e.value.name == "EPISDET_ERR_INVALID_INPUT"
+    o = oracle.search(*good, *n, order=3, score="k2", top_k=k)
+    assert_same(episdet.search(*good, *n, order=3, top_k=k, engine="tensor"), o, k)
+
+
 @pytest.mark.parametrize("score", ["k2", "mi"])
 def test_cohort_padding_bits_are_not_counted(episdet, oracle, score):
     """Set bits past the last sample, of the planes and of the labels: label mode
