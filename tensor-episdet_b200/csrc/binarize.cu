@@ -25,11 +25,12 @@ __global__ void __launch_bounds__(kListThreads) class_lists_kernel(const uint8_t
                                                                    int* __restrict__ idx, int* __restrict__ num_cases) {
     __shared__ int s_warp[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int per = (n + kListThreads - 1) / kListThreads * 32;  // samples of a warp
-    const int s0 = min(n, warp * per), s1 = min(n, s0 + per);
+    // (n may be close to 2^31: unsigned positions hold the sums past it.)
+    const uint32_t per = ((uint32_t)n + kListThreads - 1) / kListThreads * 32;  // samples of a warp
+    const uint32_t s0 = min((uint32_t)n, warp * per), s1 = min((uint32_t)n, s0 + per);
     int cnt = 0;
 #pragma unroll 8
-    for (int i = s0; i < s1; i += 32)
+    for (uint32_t i = s0; i < s1; i += 32)
         cnt += __popc(__ballot_sync(0xFFFFFFFFu, i + lane < s1 && __ldg(is_case + i + lane) != 0));
     if (lane == 0) s_warp[warp] = cnt;
     __syncthreads();
@@ -38,13 +39,13 @@ __global__ void __launch_bounds__(kListThreads) class_lists_kernel(const uint8_t
         below += i < warp ? s_warp[i] : 0;
         total += s_warp[i];
     }
-    int ic = below, in = total + s0 - below;
+    int ic = below, in = total + (int)s0 - below;
 #pragma unroll 8
-    for (int i = s0; i < s1; i += 32) {
+    for (uint32_t i = s0; i < s1; i += 32) {
         const bool here = i + lane < s1, is = here && __ldg(is_case + i + lane) != 0;
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, is), v = __ballot_sync(0xFFFFFFFFu, here);
         const uint32_t lower = (1u << lane) - 1u;
-        if (here) idx[is ? ic + __popc(m & lower) : in + __popc(~m & lower)] = i + lane;
+        if (here) idx[is ? ic + __popc(m & lower) : in + __popc(~m & lower)] = (int)i + lane;
         ic += __popc(m);
         in += __popc(v & ~m);
     }
@@ -62,10 +63,11 @@ constexpr int kBinSnps = 16;
 
 // Four samples of 16 SNPs a thread.
 __global__ void __launch_bounds__(256) pack_genotypes_kernel(const uint8_t* __restrict__ geno, int M, int n,
-                                                             uint32_t* __restrict__ packed, int pitch,
+                                                             uint32_t* __restrict__ packed, size_t pitch,
                                                              int* __restrict__ bad) {
-    const int i0 = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x), snp0 = (int)blockIdx.y * kBinSnps;
-    if (i0 >= n) return;
+    const uint32_t i0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);  // below 2^31 + 1024
+    const int snp0 = (int)blockIdx.y * kBinSnps;
+    if (i0 >= (uint32_t)n) return;
     const int ns = min(kBinSnps, M - snp0);
     uint32_t acc[4] = {0, 0, 0, 0}, over = 0;
     auto add = [&](int s, uint32_t x) {
@@ -77,7 +79,7 @@ __global__ void __launch_bounds__(256) pack_genotypes_kernel(const uint8_t* __re
     // Four bytes at any alignment are two aligned words, where those lie in the
     // matrix for all 16 rows; else one byte at a time (2 past the row's end).
     const uint8_t* first = geno + (size_t)snp0 * n + i0;
-    if (ns == kBinSnps && i0 + 4 <= n && first - geno >= 3 &&
+    if (ns == kBinSnps && i0 + 4 <= (uint32_t)n && first - geno >= 3 &&
         first + (size_t)(kBinSnps - 1) * n + 8 <= geno + (size_t)M * n) {
         uint32_t lo[kBinSnps], hi[kBinSnps];
 #pragma unroll
@@ -94,11 +96,11 @@ __global__ void __launch_bounds__(256) pack_genotypes_kernel(const uint8_t* __re
         for (int s = 0; s < ns; ++s) {
             const uint8_t* p = first + (size_t)s * n;
             uint32_t x = 0;
-            for (int e = 0; e < 4; ++e) x |= (uint32_t)(i0 + e < n ? p[e] : 2) << (8 * e);
+            for (int e = 0; e < 4; ++e) x |= (uint32_t)(i0 + e < (uint32_t)n ? p[e] : 2) << (8 * e);
             add(s, x);
         }
     }
-    *reinterpret_cast<uint4*>(packed + (size_t)blockIdx.y * pitch + i0) = make_uint4(acc[0], acc[1], acc[2], acc[3]);
+    *reinterpret_cast<uint4*>(packed + blockIdx.y * pitch + i0) = make_uint4(acc[0], acc[1], acc[2], acc[3]);
     if (over) atomicExch(bad, 1);
 }
 
@@ -110,7 +112,7 @@ struct BinClass {
     uint32_t* out;   // [M][2][W]
     int n, W;
 };
-__global__ void __launch_bounds__(256) planes_kernel(const uint32_t* __restrict__ packed, int pitch, int M, BinClass a,
+__global__ void __launch_bounds__(256) planes_kernel(const uint32_t* __restrict__ packed, size_t pitch, int M, BinClass a,
                                                      BinClass b) {
     const int lane = threadIdx.x & 31, wa = a.W / 8, wb = b.W / 8;
     const int chunk = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), snp0 = (int)blockIdx.y * kBinSnps;
@@ -120,7 +122,7 @@ __global__ void __launch_bounds__(256) planes_kernel(const uint32_t* __restrict_
     uint32_t* __restrict__ out = second ? b.out : a.out;
     const int nk = second ? b.n : a.n, W = second ? b.W : a.W;
     const int w0 = (second ? chunk - wa : chunk) * 8;
-    const uint32_t* __restrict__ p = packed + (size_t)blockIdx.y * pitch;
+    const uint32_t* __restrict__ p = packed + blockIdx.y * pitch;
     uint32_t v[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -196,14 +198,17 @@ extern "C" episdet_status episdet_binarize(const uint8_t* genotypes, int32_t num
             d_out[c] = (uint32_t*)w->bin_out[c].p;
         }
     }
-    const int groups = (M + kBinSnps - 1) / kBinSnps, pitch = (n + 3) & ~3;
+    const int groups = (int)((M + kBinSnps - 1L) / kBinSnps);
+    const size_t pitch = ((size_t)n + 3) & ~(size_t)3;
     const BinClass ca{d_idx, d_out[0], nc, Wc}, cb{d_idx + nc, d_out[1], nn, Wn};
     // SNP groups in batches of at most 64 MB of words (and of the grid's second dimension).
-    const int batch = (int)std::max<size_t>(1, std::min<size_t>(32768, ((size_t)64 << 20) / (sizeof(uint32_t) * (size_t)pitch)));
-    CUDA_TRY(w->bin_pack.ensure(sizeof(uint32_t) * (size_t)std::min(groups, batch) * pitch));
+    const int batch = (int)std::max<size_t>(1, std::min<size_t>(32768, ((size_t)64 << 20) / (sizeof(uint32_t) * pitch)));
+    CUDA_TRY(w->bin_pack.ensure(sizeof(uint32_t) * std::min(groups, batch) * pitch));
     uint32_t* d_pack = (uint32_t*)w->bin_pack.p;
     for (int g0 = 0; g0 < groups; g0 += batch) {
-        const int ng = std::min(batch, groups - g0), r0 = g0 * kBinSnps, rows = std::min(M - r0, ng * kBinSnps);
+        const int ng = std::min(batch, groups - g0);
+        const long r0 = (long)g0 * kBinSnps;
+        const int rows = (int)std::min(M - r0, (long)ng * kBinSnps);
         pack_genotypes_kernel<<<dim3((unsigned)((pitch / 4 + 255) / 256), (unsigned)ng), 256, 0, s>>>(
             d_geno + (size_t)r0 * n, rows, n, d_pack, pitch, d_flag);
         CHECK_LAUNCH();

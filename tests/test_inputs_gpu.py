@@ -100,3 +100,33 @@ def test_device_labels_still_being_written_on_the_callers_stream(episdet, oracle
         a, b, na, nb = oracle.split_by_label(planes, n, lab)
         want = oracle.search(a, b, na, nb, order=2, score="k2", top_k=k)
         assert_same(episdet._to_result(2, rs[i], keep[i]), want, k)
+
+
+def test_binarize_most_samples(episdet):
+    """2^31 - 1 samples: sample i is a case if i is odd, and sample j of either
+    class has genotype j % 3, so that the plane words repeat every three."""
+    import torch
+
+    n = 2**31 - 1
+    try:
+        i = torch.arange(n, dtype=torch.int32, device="cuda")
+        flags = (i & 1).to(torch.uint8)
+        i >>= 1
+        i %= 3
+        g = i.to(torch.uint8)[None]
+        del i
+        cases, controls, nc, nn = episdet.binarize(g, flags)
+        assert (nc, nn) == (n // 2, n - n // 2)
+        del g, flags
+        for got, k in ((cases, nc), (controls, nn)):
+            bits = (np.arange(96)[None] % 3 == np.arange(2)[:, None]).astype(np.uint32).reshape(2, 3, 32)
+            table = torch.from_numpy((bits << np.arange(31, -1, -1, dtype=np.uint32)).sum(2, dtype=np.uint32).view(np.int32))
+            w = episdet.class_words(k)
+            want = table.cuda()[:, torch.arange(w, device="cuda") % 3]
+            want[:, (k + 31) // 32:] = 0
+            if k % 32:
+                want[:, k // 32] &= -1 << (32 - k % 32)
+            assert torch.equal(got.view(2, w), want)
+    finally:
+        episdet.release_workspace(0)
+        torch.cuda.empty_cache()
