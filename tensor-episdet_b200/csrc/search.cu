@@ -59,14 +59,20 @@ cudaError_t DevBuf::ensure(size_t bytes) {
     }
     if (left == 1) return cudaErrorMemoryAllocation;
     cudaError_t e = cudaMalloc(&p, want);
-    if (e == cudaSuccess) cap = want;
+    if (e == cudaSuccess)
+        cap = want;
+    else
+        cudaGetLastError();  // reported here, not by the next launch's check
     return e;
 }
 cudaError_t HostBuf::ensure(size_t bytes) {
     if (bytes <= cap && p) return cudaSuccess;
     release();
     cudaError_t e = cudaMallocHost(&p, bytes);
-    if (e == cudaSuccess) cap = bytes;
+    if (e == cudaSuccess)
+        cap = bytes;
+    else
+        cudaGetLastError();
     return e;
 }
 void HostBuf::release() {

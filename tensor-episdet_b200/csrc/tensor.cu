@@ -633,9 +633,14 @@ static episdet_status launch_count(Workspace* w, int inst, const CUtensorMap& ta
     return EPISDET_OK;
 }
 
+// 16-byte words of one tile's drained segments.
+static size_t stash_slot(int nz, int nseg, bool wide) {
+    return (size_t)nseg * nz * (kTileA / 2) / 2 * (wide ? 2 : 1);
+}
+
 // Room for two tiles of drained segments per CTA.
 static episdet_status prepare_stash(Workspace* w, int nz, int nseg, bool wide, CountParams* p) {
-    p->stash_slot = (size_t)nseg * nz * (kTileA / 2) / 2 * (wide ? 2 : 1);
+    p->stash_slot = stash_slot(nz, nseg, wide);
     p->stash_cta = 2 * p->stash_slot;
     CUDA_TRY(w->stash.ensure(sizeof(uint4) * p->stash_cta * w->sms));
     p->stash = (uint4*)w->stash.p;
@@ -957,47 +962,71 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
     const size_t info_bytes = 256;
     const size_t xstride = (info_bytes + sizeof(int) * 4 * (size_t)max_n + 255) & ~size_t(255);
     // First SNPs of a launch: as many as give every CTA pair kGroupTiles tiles,
-    // at least kXGroup, with at most kGroupBytes of regrouped rows (or kXGroup's).
+    // at least kXGroup, with at most kGroupBytes of regrouped rows (or kXGroup's),
+    // and no more than the device has room for beside the pair table.
     const size_t member_bytes = (size_t)rows * pitch;
     int gmax = (int)std::min<size_t>(kMaxGroup, std::max<size_t>(kXGroup, kGroupBytes / member_bytes));
-    int blk_tiles = nt2 - a_first;  // A pair tiles (128 Y SNPs) per Y block
+    const int all_tiles = nt2 - a_first;
+    int blk_tiles = all_tiles;  // A pair tiles (128 Y SNPs) per Y block
+    if (o.pair_block_snps > 0) blk_tiles = std::min(blk_tiles, (o.pair_block_snps + kTileA - 1) / kTileA);
+    p.rt_ld = (M + 3) & ~3;
     {
         const size_t row_bytes = 8 * sizeof(float) * (size_t)M;  // one table row, both classes
         const size_t xrows_bytes = row_bytes * kTileA;
-        // The other buffers of the search first (their later ensure calls
-        // find them in place); the pair table gets what is left.
-        CUDA_TRY(w->frows.ensure((size_t)rows * pitch));
-        for (DevBuf& d : w->xsub) {
-            cudaError_t e = d.ensure(member_bytes * gmax);
-            if (e == cudaErrorMemoryAllocation && gmax > kXGroup) {
-                // Little memory left: the smallest launches.
-                cudaGetLastError();
-                gmax = kXGroup;
-                for (DevBuf& x : w->xsub) x.release();
-                for (DevBuf& x : w->xsub) CUDA_TRY(x.ensure(member_bytes * gmax));
-                break;
-            }
-            CUDA_TRY(e);
-        }
-        for (int c = 0; c < 2; ++c)
-            CUDA_TRY(w->planes_t[c].ensure(sizeof(uint32_t) * (size_t)D.W[c] * 32 * tt_row_words(rows)));
-        CUDA_TRY(w->xinfo.ensure((size_t)kXSets * gmax * xstride));
-        p.rt_ld = (M + 3) & ~3;
-        CUDA_TRY(w->rtab.ensure(sizeof(float2) * 9 * (size_t)p.rt_ld * gmax));
-        st = prepare_stash(w, nz, 4, (int64_t)D.n[0] + D.n[1] > 131070 || counts_wide(D.n[0], D.n[1]), &p);
-        if (st != EPISDET_OK) return st;
-        if (o.pair_block_snps > 0) {
-            blk_tiles = std::min(blk_tiles, (o.pair_block_snps + kTileA - 1) / kTileA);
-        } else if (w->ptab.cap < row_bytes * (size_t)M) {
-            // (Asked for only when the table has to grow: on some hosts the
-            // driver takes 9 ms to answer, more than a small search.)
+        const bool wide = counts_wide(D.n[0], D.n[1]);
+        // The buffers of the search but for the pair table.
+        struct Need {
+            DevBuf* buf;
+            size_t bytes;
+        };
+        auto needs = [&](int g) {
+            std::vector<Need> v = {{&w->frows, (size_t)rows * pitch},
+                                   {&w->xinfo, (size_t)kXSets * g * xstride},
+                                   {&w->rtab, sizeof(float2) * 9 * (size_t)p.rt_ld * g},
+                                   {&w->stash, sizeof(uint4) * 2 * stash_slot(nz, 4, wide) * w->sms}};
+            for (DevBuf& d : w->xsub) v.push_back({&d, member_bytes * g});
+            for (int c = 0; c < 2; ++c)
+                v.push_back({&w->planes_t[c], sizeof(uint32_t) * (size_t)D.W[c] * 32 * tt_row_words(rows)});
+            return v;
+        };
+        // Device memory they still take (a buffer is replaced when it grows).
+        auto growth = [&](int g) {
+            size_t more = 0;
+            for (const Need& d : needs(g)) more += d.bytes > d.buf->cap ? d.bytes - d.buf->cap : 0;
+            return more;
+        };
+        auto table_bytes = [&] { return row_bytes * (blk_tiles < all_tiles ? (size_t)blk_tiles * kTileA : (size_t)M); };
+        // Chooses gmax and, unless asked for, the pair table's blocks.  (Free
+        // memory is asked for only when something has to grow: on some hosts the
+        // driver takes 9 ms to answer, more than a small search.)
+        auto plan = [&]() -> episdet_status {
+            const bool asked = blk_tiles < all_tiles;
+            const bool held_all = w->ptab.cap >= table_bytes() && (!asked || w->ptabx.cap >= xrows_bytes);
+            if (held_all && growth(gmax) == 0) return EPISDET_OK;
             size_t fr = 0, tot = 0;
             CUDA_TRY(cudaMemGetInfo(&fr, &tot));
             // Left for the tile lists, slots, merge buffers and the driver.
             const size_t reserve = std::max<size_t>(tot / 32, (size_t)1 << 30);
+            const size_t table = held_all ? 0 : table_bytes() + (asked ? xrows_bytes : 0);
             // The pair-table buffers are replaced when they grow, so their memory counts as free.
-            const size_t held = w->ptab.cap + w->ptabx.cap;
-            const size_t avail = fr + held > reserve ? fr + held - reserve : 0;
+            size_t held = held_all ? 0 : w->ptab.cap + w->ptabx.cap;
+            const size_t least = reserve + table + growth(kXGroup);
+            if (fr + held >= least) {
+                // Larger launches take a small part of what is left, so that they
+                // narrow nothing for the other lanes of a batch or other processes.
+                const size_t spare = (fr + held - least) / 16;
+                while (gmax > kXGroup && growth(gmax) > growth(kXGroup) + spare) gmax = std::max(kXGroup, gmax * 3 / 4);
+                return EPISDET_OK;
+            }
+            // Little memory left: the smallest launches, and what earlier searches'
+            // larger ones hold goes back.
+            gmax = kXGroup;
+            for (const Need& d : needs(gmax))
+                if (d.buf->cap > d.bytes) d.buf->release();
+            if (asked || held_all) return EPISDET_OK;
+            CUDA_TRY(cudaMemGetInfo(&fr, &tot));
+            const size_t taken = reserve + growth(gmax);
+            const size_t avail = fr + held > taken ? fr + held - taken : 0;
             if (row_bytes * (size_t)M > avail) {
                 const size_t left = avail > xrows_bytes ? avail - xrows_bytes : 0;
                 blk_tiles = (int)std::min<size_t>((size_t)blk_tiles, left / (row_bytes * kTileA));
@@ -1007,10 +1036,35 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
                                      "left beside the operand buffers",
                                      M, (double)avail / 1e9);
             }
+            return EPISDET_OK;
+        };
+        auto allocate = [&]() -> cudaError_t {
+            for (const Need& d : needs(gmax)) {
+                const cudaError_t e = d.buf->ensure(d.bytes);
+                if (e != cudaSuccess) return e;
+            }
+            // (A table that grows takes the memory of the buffer it no longer needs.)
+            const bool blocked = blk_tiles < all_tiles;
+            if (!blocked && w->ptab.cap < table_bytes()) w->ptabx.release();
+            if (blocked && w->ptabx.cap < xrows_bytes && w->ptab.cap > table_bytes()) w->ptab.release();
+            cudaError_t e = w->ptab.ensure(table_bytes());
+            if (e == cudaSuccess && blocked) e = w->ptabx.ensure(xrows_bytes);
+            return e;
+        };
+        for (;;) {
+            st = plan();
+            if (st != EPISDET_OK) return st;
+            const cudaError_t e = allocate();
+            if (e == cudaSuccess) break;
+            if (e != cudaErrorMemoryAllocation || gmax == kXGroup) return cuda_fail(e, "3-way search buffers");
+            // Less memory than it seemed (another lane or process): once more with
+            // the smallest launches.
+            gmax = kXGroup;
+            for (const Need& d : needs(gmax))
+                if (d.buf->cap > d.bytes) d.buf->release();
         }
-        const bool blocked = blk_tiles < nt2 - a_first;
-        CUDA_TRY(w->ptab.ensure(row_bytes * (blocked ? (size_t)blk_tiles * kTileA : (size_t)M)));
-        if (blocked) CUDA_TRY(w->ptabx.ensure(xrows_bytes));
+        st = prepare_stash(w, nz, 4, wide, &p);
+        if (st != EPISDET_OK) return st;
     }
     const bool blocked = blk_tiles < nt2 - a_first;
     const int nblk = (nt2 - a_first + blk_tiles - 1) / blk_tiles;
