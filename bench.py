@@ -272,8 +272,7 @@ def batched_vs_plain(reps=2):
             "ratio": min(tp) / min(tb), "identical": same,
             "plain_rate": work / min(tp) / 1e12, "batched_rate": work / min(tb) / 1e12, "unit": UNIT,
             "batched_autotune": True,
-            "tuned_wide": sorted({(nc_ if nc_ < nn_ else nn_).bit_length() - 1: episdet.tuned_stage(3, "k2", nc_, nn_)
-                                    for _, _, nc_, nn_, _, o_ in co if o_ == 3}.items()),
+            "tuned_wide": [(m, nc + nn, episdet.tuned_tiles(3, "k2", m, nc, nn)) for _, _, nc, nn, m, o in co if o == 3],
             "timing": f"wall clock per pass, device-resident planes, best of {reps} after a warm-up pass"}
 
 

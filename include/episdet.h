@@ -67,11 +67,11 @@ enum { EPISDET_ENGINE_AUTO = 0, EPISDET_ENGINE_TENSOR = 1, EPISDET_ENGINE_SIMT =
 #define EPISDET_FLAG_NO_VALIDATE 0x2u  /* skip the padding / plane-overlap check */
 #define EPISDET_FLAG_TIMING 0x4u       /* time every counting-kernel launch (result.count_kernel_ms) */
 /* Pick the triplet kernel instance for this shape by measurement: the first
- * search of a shape (order, score, log2 of the smaller class) times the
- * instances with wide (112) and narrow (56 third SNPs) tiles on the first 8
- * first SNPs of its own data and keeps the faster; the choice is cached for
- * the process and, when the environment variable EPISDET_TUNE_CACHE names a
- * file, read from and appended to it.  Without the flag the instance follows
+ * search of a shape (order, score, log2 of the smaller class, log2 of the SNPs
+ * in halves) times the instances with wide (112) and narrow (56 third SNPs)
+ * tiles on the first 8 first SNPs of its own data and keeps the faster; the
+ * choice is cached for the process and, when the environment variable
+ * EPISDET_TUNE_CACHE names a file, read from and appended to it.  Without the flag the instance follows
  * a fixed rule (narrow tiles for panels of few SNPs).  Results are the same
  * either way. */
 #define EPISDET_FLAG_AUTOTUNE 0x8u
@@ -273,7 +273,10 @@ episdet_status episdet_generate_labels(uint64_t seed, int32_t num_samples, int32
                                        uint32_t* labels);
 
 /* The cached EPISDET_FLAG_AUTOTUNE choice for a shape: 1 = wide triplet
- * tiles, 0 = narrow ones, -1 = not tuned yet. */
+ * tiles, 0 = narrow ones, -1 = not tuned yet.  episdet_tuned_stage: the newest
+ * choice for these class sizes, whatever the number of SNPs was. */
+int32_t episdet_tuned_tiles(int32_t order, int32_t score, int32_t num_snps, int32_t num_cases,
+                            int32_t num_controls);
 int32_t episdet_tuned_stage(int32_t order, int32_t score, int32_t num_cases, int32_t num_controls);
 
 uint64_t episdet_n_choose_k(uint32_t n, uint32_t k);

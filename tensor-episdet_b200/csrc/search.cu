@@ -521,16 +521,36 @@ namespace episdet {
 // ------------------------------------------------------------ autotuning
 // The measured choice of triplet instance per shape (EPISDET_FLAG_AUTOTUNE),
 // kept for the process and, when EPISDET_TUNE_CACHE names a file, read from it
-// once and appended to it: one "order score bucket choice" line per shape,
-// bucket = floor(log2(smaller class)).
+// once and appended to it: one "order score bucket choice" line per shape, the
+// bucket floor(log2(smaller class)) + 32 x the panel's size class.  Which tile
+// width is faster depends on both: on the panel by how full the last tiles of
+// its rows are, on the samples by whether the scoring or the operand reads
+// bound (512 to 704 SNPs: narrow up to 4 % faster at 4,000 samples, 8 to 10 %
+// slower at 262,144).
 static std::mutex g_tune_mu;
-static std::map<int, int> g_tune;
+static std::map<int, int> g_tune;       // by tune_key
+static std::map<int, int> g_tune_last;  // by tune_key without the panel: the newest of any panel
 static bool g_tune_loaded = false;
 
-static int tune_key(int order, int score, int nc, int nn) {
+// 0 below 128 SNPs (one row of tiles, the widths within 7 % of each other; the
+// lines of files written without panel classes are these), then 1, 2, ... from each power of sqrt 2 on: [128, 181],
+// [182, 255], ...
+static int panel_class(int64_t M) {
+    int c = 0;
+    while (M * M >= (int64_t)1 << (14 + c)) ++c;
+    return c;
+}
+
+static int tune_key(int order, int score, int nc, int nn, int panel) {
     int m = std::max(1, std::min(nc, nn)), b = 0;
     while (m >>= 1) ++b;
-    return (order << 16) | (score << 8) | b;
+    return (order << 24) | (score << 16) | (32 * panel + b);
+}
+static int tune_key_any(int key) { return key & ~0xFFE0; }
+
+static void tune_put_locked(int key, int choice) {
+    g_tune[key] = choice;
+    g_tune_last[tune_key_any(key)] = choice;
 }
 
 static void tune_load_locked() {
@@ -543,26 +563,26 @@ static void tune_load_locked() {
     while (std::fgets(line, sizeof(line), f)) {
         int order, score, bucket, choice;
         if (std::sscanf(line, "%d %d %d %d", &order, &score, &bucket, &choice) == 4 && (choice == 0 || choice == 1) &&
-            order >= 2 && order <= 3 && score >= 0 && score <= 1 && bucket >= 0 && bucket < 64)
-            g_tune[(order << 16) | (score << 8) | bucket] = choice;
+            order >= 2 && order <= 3 && score >= 0 && score <= 1 && bucket >= 0 && bucket < 32 * 32)
+            tune_put_locked((order << 24) | (score << 16) | bucket, choice);
     }
     std::fclose(f);
 }
 
-static int tune_lookup(int key) {
+static int tune_lookup(const std::map<int, int>& t, int key) {
     std::lock_guard<std::mutex> g(g_tune_mu);
     tune_load_locked();
-    auto it = g_tune.find(key);
-    return it == g_tune.end() ? -1 : it->second;
+    auto it = t.find(key);
+    return it == t.end() ? -1 : it->second;
 }
 
 static void tune_store(int key, int choice) {
     std::lock_guard<std::mutex> g(g_tune_mu);
     tune_load_locked();
-    g_tune[key] = choice;
+    tune_put_locked(key, choice);
     const char* path = std::getenv("EPISDET_TUNE_CACHE");
     if (FILE* f = path && *path ? std::fopen(path, "a") : nullptr) {
-        std::fprintf(f, "%d %d %d %d\n", key >> 16, (key >> 8) & 0xFF, key & 0xFF, choice);
+        std::fprintf(f, "%d %d %d %d\n", key >> 24, (key >> 16) & 0xFF, key & 0xFFFF, choice);
         std::fclose(f);
     }
 }
@@ -617,8 +637,8 @@ episdet_status search_locked(Workspace* w, const episdet_dataset* data, const ep
     if (st0 != EPISDET_OK) return st0;
     const bool simt = o.engine == EPISDET_ENGINE_SIMT || !tensor_exact_for(data);
     if ((o.flags & EPISDET_FLAG_AUTOTUNE) && o.order == 3 && !simt) {
-        const int key = tune_key(o.order, o.score, data->num_cases, data->num_controls);
-        int choice = tune_lookup(key);
+        const int key = tune_key(o.order, o.score, data->num_cases, data->num_controls, panel_class(data->num_snps));
+        int choice = tune_lookup(g_tune, key);
         if (choice < 0) {
             episdet_status st = tune_probe(w, data, o, &choice);
             if (st != EPISDET_OK) return st;
@@ -753,5 +773,11 @@ extern "C" int64_t episdet_last_launch_profile(int32_t device, double* ms, doubl
 extern "C" void episdet_test_fail_allocation(int32_t after) { episdet::g_fail_alloc.store(after > 0 ? after : 0); }
 
 extern "C" int32_t episdet_tuned_stage(int32_t order, int32_t score, int32_t num_cases, int32_t num_controls) {
-    return episdet::tune_lookup(episdet::tune_key(order, score, num_cases, num_controls));
+    return episdet::tune_lookup(episdet::g_tune_last, episdet::tune_key(order, score, num_cases, num_controls, 0));
+}
+
+extern "C" int32_t episdet_tuned_tiles(int32_t order, int32_t score, int32_t num_snps, int32_t num_cases,
+                                       int32_t num_controls) {
+    const int panel = episdet::panel_class(std::min<int64_t>(std::max(num_snps, 0), 1 << 21));
+    return episdet::tune_lookup(episdet::g_tune, episdet::tune_key(order, score, num_cases, num_controls, panel));
 }

@@ -48,7 +48,7 @@ EXPORTED = [
     "episdet_generate", "episdet_generate_cohort", "episdet_generate_labels", "episdet_n_choose_k",
     "episdet_status_string", "episdet_last_error", "episdet_abi_version", "episdet_release_workspace",
     "episdet_search_pairs_noalloc", "episdet_binarize", "episdet_perm_pvalues", "episdet_search_resumable",
-    "episdet_tuned_stage", "episdet_test_fail_allocation", "episdet_last_launch_profile",
+    "episdet_tuned_stage", "episdet_tuned_tiles", "episdet_test_fail_allocation", "episdet_last_launch_profile",
 ]
 
 
@@ -397,9 +397,16 @@ def test_fail_allocation(after: int) -> None:
     lib().episdet_test_fail_allocation(after)
 
 
-def tuned_stage(order: int, score, num_cases: int, num_controls: int) -> int:
+def tuned_tiles(order: int, score, num_snps: int, num_cases: int, num_controls: int) -> int:
     """The cached FLAG_AUTOTUNE choice for a shape: 1 wide triplet tiles,
     0 narrow ones, -1 not tuned yet."""
+    sc = {"k2": SCORE_K2, "mi": SCORE_MI}[score] if isinstance(score, str) else int(score)
+    return int(lib().episdet_tuned_tiles(order, sc, num_snps, num_cases, num_controls))
+
+
+def tuned_stage(order: int, score, num_cases: int, num_controls: int) -> int:
+    """The newest of these choices for the class sizes, whatever the number of
+    SNPs was."""
     sc = {"k2": SCORE_K2, "mi": SCORE_MI}[score] if isinstance(score, str) else int(score)
     return int(lib().episdet_tuned_stage(order, sc, num_cases, num_controls))
 

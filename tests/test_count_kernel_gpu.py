@@ -62,6 +62,12 @@ def test_autotune_keeps_the_answer(episdet, oracle):
     assert episdet.tuned_stage(3, "k2", 2000, 2100) in (0, 1)
 
 
+def test_autotuned_choice_is_for_its_panel_size(episdet, oracle):
+    check(episdet, oracle, 3, 100, 600, 500, "k2", 100, flags=(episdet.FLAG_AUTOTUNE,))
+    assert episdet.tuned_tiles(3, "k2", 100, 600, 500) in (0, 1)
+    assert episdet.tuned_tiles(3, "k2", 1500, 600, 500) == -1
+
+
 def test_permutations_device_labels_and_unaligned_planes(episdet, oracle):
     """Label mode takes labels and planes of either memory; planes that are not
     16-byte aligned go through the per-label split.  Same answers."""

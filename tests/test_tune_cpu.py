@@ -1,6 +1,7 @@
 """The EPISDET_FLAG_AUTOTUNE cache on the CPU: the file named by
 EPISDET_TUNE_CACHE is read once per process ("order score bucket choice"
-lines, bucket = floor(log2(smaller class))); malformed lines are skipped.
+lines, bucket = floor(log2(smaller class)) + 32 x the panel's size class);
+malformed lines are skipped.
 Each case runs in a fresh process, since the cache is loaded once."""
 import os
 import subprocess
@@ -32,3 +33,17 @@ def test_cache_file_is_read(tmp_path):
 
 def test_missing_cache_file_means_untuned(tmp_path):
     assert _query(tmp_path / "absent.txt", [(3, "k2", 70000, 66000)]) == [-1]
+
+
+def test_a_choice_is_for_its_panel_size(tmp_path):
+    cache = tmp_path / "tune.txt"
+    cache.write_text("3 0 14 0\n3 0 174 0\n3 0 270 1\n3 0 1039 1\n")
+    # 14 + 32 x {0: below 128 SNPs, 5: [512, 724], 8: [1449, 2047]}; 1039 is past every class
+    panels = [3, 127, 128, 511, 512, 724, 725, 1448, 1449, 2047, 2048, 2097151]
+    code = ("import sys; sys.path.insert(0, %r); import episdet; "
+            "print([episdet.tuned_tiles(3, 'k2', m, 20000, 30000) for m in %r], "
+            "episdet.tuned_stage(3, 'k2', 20000, 30000))" % (PKG, panels))
+    p = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120,
+                       env=dict(os.environ, EPISDET_TUNE_CACHE=str(cache)))
+    assert p.returncode == 0, p.stderr
+    assert p.stdout.strip() == "[0, 0, -1, -1, 0, 0, -1, -1, 1, 1, -1, -1] 1"
