@@ -248,17 +248,30 @@ extern "C" episdet_status episdet_search_perm(const episdet_cohort* cohort, cons
     // Label mode: the cohort's transposed planes, genotype counts and pair
     // totals, once, shared read-only by every lane (the computation ends with a
     // synchronise of lane 0's stream).
-    LabelCohort lc{d_planes, M, n, W, nullptr, nullptr, nullptr};
     const size_t tot_bytes = sizeof(float4) * (size_t)M * (size_t)M;
-    const bool label_mode = o.order == 2 && o.engine != EPISDET_ENGINE_SIMT && !(o.flags & EPISDET_FLAG_PERM_SPLIT) &&
-                            n <= kTensorMaxClass && tot_bytes <= (size_t)kLabelTotalsMaxBytes &&
-                            ((uintptr_t)d_planes & 15) == 0;  // its kernels read 16 bytes at a time
+    bool label_mode = o.order == 2 && o.engine != EPISDET_ENGINE_SIMT && !(o.flags & EPISDET_FLAG_PERM_SPLIT) &&
+                      n <= kTensorMaxClass && tot_bytes <= (size_t)kLabelTotalsMaxBytes;
+    begin_call(w0, o);
+    if (label_mode && ((uintptr_t)d_planes & 15) != 0) {
+        // Its kernels read 16 bytes at a time: an aligned copy of the planes, or
+        // (no room for one) the per-label split.
+        const cudaError_t e = w0->perm_planes.ensure(sizeof(uint32_t) * plane_words);
+        if (e == cudaSuccess) {
+            CUDA_TRY(cudaMemcpyAsync(w0->perm_planes.p, d_planes, sizeof(uint32_t) * plane_words,
+                                     cudaMemcpyDeviceToDevice, w0->st));
+            d_planes = (const uint32_t*)w0->perm_planes.p;
+        } else if (e == cudaErrorMemoryAllocation) {
+            label_mode = false;
+        } else {
+            CUDA_TRY(e);
+        }
+    }
+    LabelCohort lc{d_planes, M, n, W, nullptr, nullptr, nullptr};
     const uint32_t* d_labels = labels;
     std::vector<uint32_t> h_labels;
     if (label_mode) {
-        // On the call's stream: device labels may still be on their way there.
-        begin_call(w0, o);
-        // The labels on both sides: the host counts their cases.
+        // The labels on both sides (the host counts their cases), copied on the
+        // call's stream: device labels may still be on their way there.
         const size_t words = (size_t)num_labels * W;
         if (on_device) {
             h_labels.resize(words);

@@ -130,3 +130,30 @@ def test_binarize_most_samples(episdet):
     finally:
         episdet.release_workspace(0)
         torch.cuda.empty_cache()
+
+
+def test_unaligned_cohort_planes_run_in_label_mode(episdet, oracle):
+    """4-byte aligned planes are copied; without room for the copy every label is
+    split, with the same answers."""
+    import torch
+
+    n, M, nc, nl, k = 2085, 150, 700, 2, 40
+    planes = episdet.generate_cohort(77, M, n)
+    labels = episdet.generate_labels(78, n, nc, nl)
+    dev = torch.from_numpy(planes.view(np.int32)).cuda()
+    shifted = torch.zeros(dev.numel() + 1, dtype=torch.int32, device="cuda")
+    shifted[1:] = dev.flatten()
+    off = shifted[1:].view(dev.shape)
+    dl = torch.from_numpy(labels.view(np.int32)).cuda()
+    torch.cuda.synchronize()
+    assert off.data_ptr() % 16 == 4
+    aligned = episdet.search_perm(dev, n, dl, top_k=k)
+    split = episdet.search_perm(dev, n, dl, top_k=k, flags=episdet.FLAG_PERM_SPLIT)
+    assert aligned[0].kernel_launches != split[0].kernel_launches
+    for fail, same in ((0, aligned), (1, split)):
+        episdet.release_workspace(0)
+        episdet.test_fail_allocation(fail)
+        for r, a, s in zip(episdet.search_perm(off, n, dl, top_k=k), aligned, same):
+            assert r.kernel_launches == s.kernel_launches
+            assert r.snps == a.snps and np.array_equal(r.top_snps, a.top_snps)
+            assert np.array_equal(r.top_fp32, a.top_fp32) and np.array_equal(r.top_fp64, a.top_fp64)
