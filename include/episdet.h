@@ -72,7 +72,7 @@ enum { EPISDET_ENGINE_AUTO = 0, EPISDET_ENGINE_TENSOR = 1, EPISDET_ENGINE_SIMT =
  * tiles on the first 8 first SNPs of its own data and keeps the faster; the
  * choice is cached for the process and, when the environment variable
  * EPISDET_TUNE_CACHE names a file, read from and appended to it.  Without the flag the instance follows
- * a fixed rule (narrow tiles for panels of few SNPs).  Results are the same
+ * a fixed rule (narrow tiles for few SNPs and few samples).  Results are the same
  * either way. */
 #define EPISDET_FLAG_AUTOTUNE 0x8u
 /* Testing aid for failure detection: the tensor engine's scoring warps first

@@ -56,10 +56,20 @@ constexpr int kXGroup = 4;  // first SNPs per triplet launch at least
 // samples: 8 39.8 ms, 16 39.0, 32 38.7 at twice the rows).
 constexpr int kGroupTiles = 16;
 constexpr size_t kGroupBytes = (size_t)2 << 30;   // regrouped rows a launch may take for them
-// Panels up to this size use narrow triplet tiles (the last wide tile of a row
-// is a large share of theirs): 256 SNPs x 4096 samples 0.73 ms narrow, 0.83
-// wide; 600 x 10007 3.01 and 3.11; 1536 x 40000 42.0 and 37.8.
+// Panels up to this size use narrow triplet tiles, whose last tile of a row is a
+// smaller share of the work, up to a number of samples: past it a tile takes as
+// long as its MMAs, and a narrow one's need 103 operand bytes a clock instead of
+// 67.  Narrow against wide, K2, ms:
+//   samples     4,000        40,000       56,000        90,000       262,144
+//   200 SNPs    0.61  0.62   0.94  0.97    1.13  1.13    1.55  1.47    3.9   3.6
+//   400         1.44  1.39   2.51  2.35    3.20  2.83    4.71  4.06   13.0  10.9
+//   600         2.82  2.92   5.04  5.00    6.51  6.19    9.98  9.39   28.2  25.6
+//   704         4.10  4.14   7.01  7.14    9.04  8.68   13.90 13.26   37.8  34.5
+//   1024       10.54 10.20  15.57 15.90                               83.5  74.2
+//   1250       18.22 17.44  25.63 25.94
+// (MI the same within 3 %; above 704 SNPs neither is ahead at few samples.)
 constexpr int kNarrowTileSnps = 704;
+constexpr int kNarrowTileSamples = 48000;
 
 struct Workspace {
     int device = 0;

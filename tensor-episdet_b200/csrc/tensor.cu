@@ -938,9 +938,11 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
     const int Kc = D.W[0] * 32, Kn = D.W[1] * 32;
     const int rows = 2 * M;
     const int bs_lines = (M + 255) / 256;
-    // Triplet tiles: narrow for panels of few B tiles, whose last tile is a
-    // large share of the work (w->stage_override: the autotuner's choice).
-    const bool narrow = w->stage_override >= 0 ? w->stage_override == 0 : M <= kNarrowTileSnps;
+    // Triplet tiles: narrow for panels of few B tiles and few samples
+    // (w->stage_override: the autotuner's choice).
+    const bool narrow = w->stage_override >= 0
+                            ? w->stage_override == 0
+                            : M <= kNarrowTileSnps && D.n[0] + D.n[1] <= kNarrowTileSamples;
     const int nz = narrow ? kNarrowZ : kWideZ;
     const int inst = kITriplets + 2 * T.score + (narrow ? 1 : 0);
 

@@ -1,7 +1,7 @@
 """The counting kernel at the edges of its tiles, against the oracle.
 
 Tiles are 128 A SNPs x 112 (wide) or 56 (narrow) B SNPs; panels of up to 704
-SNPs run narrow triplet tiles, pairs run narrow tiles when wide ones are fewer
+SNPs and 48,000 samples run narrow triplet tiles, pairs run narrow tiles when wide ones are fewer
 than the CTA pairs.  Counts pass through a buffer of 16-bit values, or 32-bit
 ones for a first SNP with a kept genotype of more than 65,535 samples.  K is
 cut in blocks of 256 samples per segment.  Everything is exact, so the bar is
@@ -35,6 +35,44 @@ def test_tile_edges(episdet, oracle, order, M, score):
 @pytest.mark.parametrize("M,slab", [(704, (696, 0)), (705, (0, 1)), (705, (126, 129)), (784, (330, 336))])
 def test_triplet_tile_widths_and_list_edges(episdet, oracle, M, slab, score):
     check(episdet, oracle, 3, M, 1300, 900, score, 1536, slab=slab)
+
+
+def test_narrow_tiles_with_counts_past_16_bits(tmp_path):
+    """Reached by an autotuned choice only (here from a cache file)."""
+    import os
+    import subprocess
+    import sys
+
+    import episdet as e
+
+    cache = tmp_path / "tune.txt"
+    cache.write_text("3 0 17 0\n")
+    code = f"""
+import sys
+sys.path.insert(0, {os.path.dirname(e.__file__)!r})
+import numpy as np, episdet
+n = (170000, 150000)
+data = episdet.generate(11, 40, *n, maf=(0.3, 0.36))
+wide, narrow = (episdet.search(*data, *n, order=3, top_k=64, engine="tensor", flags=f | episdet.FLAG_TIMING)
+                for f in (0, episdet.FLAG_AUTOTUNE))
+assert 1.9 < wide.executed_macs / narrow.executed_macs < 2.1
+assert np.array_equal(wide.top_snps, narrow.top_snps) and np.array_equal(wide.top_fp64, narrow.top_fp64)
+assert np.array_equal(wide.top_fp32.view(np.uint32), narrow.top_fp32.view(np.uint32))
+"""
+    p = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, EPISDET_TUNE_CACHE=str(cache)))
+    assert p.returncode == 0, p.stderr
+
+
+def test_tile_width_follows_the_samples_too(episdet, oracle):
+    """40 SNPs are one tile of either width: a wide one issues twice the MACs."""
+    M, k, macs = 40, 64, []
+    for nn in (24000, 24001):
+        cases, controls = episdet.generate(5, M, 24000, nn, maf=(0.3, 0.36))
+        r = episdet.search(cases, controls, 24000, nn, order=3, top_k=k, engine="tensor", flags=episdet.FLAG_TIMING)
+        assert_same(r, oracle.search(cases, controls, 24000, nn, order=3, score="k2", top_k=k), k)
+        macs.append(r.executed_macs)
+    assert 1.9 < macs[1] / macs[0] < 2.1
 
 
 @pytest.mark.parametrize("order,M,slab", [(3, 24, (0, 0)), (3, 710, (3, 4)), (2, 40, (0, 0)), (2, 1500, (700, 703))])
