@@ -301,6 +301,14 @@ int64_t episdet_last_launch_profile(int32_t device, double* ms, double* macs, in
  * after <= 0 disarms it. */
 void episdet_test_fail_allocation(int32_t after);
 
+/* Testing aid -- no counterpart in the reference: the score bound's
+ * coefficients {cut_mul, cut_add, seed_mul, seed_add} for a search of this
+ * order, score and class sizes (each at least 1; no GPU needed).  With L the
+ * bound's sum in FP32, a set scoring s has L >= s * cut_mul + cut_add and scores
+ * at least as well as (L + seed_add) * seed_mul. */
+void episdet_test_bound_coefficients(int32_t order, int32_t score, int32_t num_cases, int32_t num_controls,
+                                     double* out);
+
 /* Pairs search that allocates nothing -- no counterpart in the reference.
  * For callers that cannot let a library allocate device memory: a process
  * whose memory pool or caching allocator already holds the GPU's memory, or a

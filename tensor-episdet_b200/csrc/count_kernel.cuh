@@ -208,8 +208,9 @@ __device__ __forceinline__ int group_of(const CountParams& P, int t) {
 //   ln v! = z ln z - z + ln(2 pi) / 2 - e(v), z = v + 1/2,
 // with e positive and decreasing, and e(n) + e(m) - e(n + m + 1) > 0, so
 //   score >= -(ln 2 L + 27 or 9 cells x (1/2 + ln(2 pi) / 2)),
-// too small by at most 0.1175 a cell.  A set is scored exactly only if this
-// bound, less the rounding of both sums (filter_coefficients), does not rule
+// too small by at most 0.1176 a cell (2 e(0) - e(1) = 0.11759).  A set is scored
+// exactly only if this bound, less the rounding of both sums (bound_coefficients
+// in tensor.cu, checked against scores by tests/test_score_bound_cpu.py), does not rule
 // it out of the list.  27 x 3 logarithms on the MUFU pipe bound the scoring: 8
 // clocks a warp instruction, 648 of the 32 triplets' clocks on an SM quarter.
 using f2 = unsigned long long;  // (cases, controls)

@@ -506,12 +506,12 @@ using namespace tc;
 // sum at most sum of the |b_c|.  FP32 MI: p's two roundings and the table's
 // against an entropy of at most lg 54, 81 multiply-adds on partial sums of at
 // most that.
-static void bound_coefficients(const ScoreTables& T, int nc, int nn, int cells, CountParams* p) {
+static void bound_coefficients(int score, double hy64, int nc, int nn, int cells, CountParams* p) {
     const double u = std::ldexp(1.0, -24), N = (double)nc + nn, Np = N + 1.5 * cells, ln2 = std::log(2.0);
     const double lgN = std::log2(N + 2.0);
     const double dl = std::ldexp(1.0, -22) * std::max(1.0, lgN);
     const double r = (2.0 * dl * Np + u * Np * (1.1 * cells + 4.0) + u * cells * cells * lgN + 0.5 * cells * dl) * 1.05;
-    if (T.score == EPISDET_SCORE_K2) {
+    if (score == EPISDET_SCORE_K2) {
         const double lg = std::lgamma(nc + 1.0) + std::lgamma(nn + 1.0);
         const double bt = N * ln2 + cells * (std::log(N + 2.0) + 3.0);
         const double s32 = u * (2.0 * lg + std::lgamma(N + 2.0 * cells + 2.0) + (cells + 1.0) * bt) * 1.05;
@@ -525,9 +525,9 @@ static void bound_coefficients(const ScoreTables& T, int nc, int nn, int cells, 
         const double s32 = u * (2.0 * (lgN + 1.5) + 2.0 * 12.0 + 3.0 * cells * 6.0 + 16.0);
         const double margin = r / N + s32 + 1e-7;
         p->cut_mul = N;
-        p->cut_add = -(margin + T.hy64) * N;
+        p->cut_add = -(margin + hy64) * N;
         p->seed_mul = 1.0 / N;
-        p->seed_add = (T.hy64 - margin) * N;
+        p->seed_add = (hy64 - margin) * N;
     }
 }
 
@@ -931,7 +931,7 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
     // past that are scored exactly throughout.
     p.filter = (o.flags & EPISDET_FLAG_FILTER_OFF) == 0 && std::max(D.n[0], D.n[1]) <= (1 << 22);
     p.tab_off = p.filter && T.score == EPISDET_SCORE_K2 ? 3.0f * kCellOff<0> : 0.0f;
-    bound_coefficients(T, D.n[0], D.n[1], o.order == 2 ? 9 : 27, &p);
+    bound_coefficients(T.score, T.hy64, D.n[0], D.n[1], o.order == 2 ? 9 : 27, &p);
 
     if (o.order == 2) return run_pairs(w, D, o, fb, fe, p, launches, progress);
 
@@ -1304,3 +1304,12 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
 }
 
 }  // namespace episdet
+
+extern "C" void episdet_test_bound_coefficients(int32_t order, int32_t score, int32_t num_cases, int32_t num_controls,
+                                                double* out) {
+    const double n = (double)num_cases + num_controls, a = num_cases / n, b = num_controls / n;
+    episdet::tc::CountParams p;
+    episdet::bound_coefficients(score, -a * std::log2(a) - b * std::log2(b), num_cases, num_controls,
+                                order == 2 ? 9 : 27, &p);
+    out[0] = p.cut_mul, out[1] = p.cut_add, out[2] = p.seed_mul, out[3] = p.seed_add;
+}

@@ -48,7 +48,7 @@ EXPORTED = [
     "episdet_generate", "episdet_generate_cohort", "episdet_generate_labels", "episdet_n_choose_k",
     "episdet_status_string", "episdet_last_error", "episdet_abi_version", "episdet_release_workspace",
     "episdet_search_pairs_noalloc", "episdet_binarize", "episdet_perm_pvalues", "episdet_search_resumable",
-    "episdet_tuned_stage", "episdet_tuned_tiles", "episdet_test_fail_allocation", "episdet_last_launch_profile",
+    "episdet_tuned_stage", "episdet_tuned_tiles", "episdet_test_fail_allocation", "episdet_test_bound_coefficients", "episdet_last_launch_profile",
 ]
 
 
@@ -151,6 +151,8 @@ def lib() -> ctypes.CDLL:
     L.episdet_last_launch_profile.restype = ctypes.c_int64
     L.episdet_test_fail_allocation.argtypes = [ctypes.c_int32]
     L.episdet_test_fail_allocation.restype = None
+    L.episdet_test_bound_coefficients.argtypes = [ctypes.c_int32] * 4 + [P(ctypes.c_double)]
+    L.episdet_test_bound_coefficients.restype = None
     L.episdet_search_pairs_noalloc.argtypes = [P(Dataset), P(Options), P(Result)]
     L.episdet_search_pairs_noalloc.restype = ctypes.c_int
     _lib = L
