@@ -83,8 +83,9 @@ enum { EPISDET_ENGINE_AUTO = 0, EPISDET_ENGINE_TENSOR = 1, EPISDET_ENGINE_SIMT =
 #define EPISDET_FLAG_INJECT_STALL 0x10u
 /* Searches on the tensor engine bound each set's score without table reads
  * and score exactly only the sets that can still enter the top-k list (same
- * results either way).  FILTER_OFF scores every set exactly; FILTER_ON, the
- * default, is the bound (classes past 2^22 samples are scored exactly). */
+ * results either way; classes past 2^22 samples are scored exactly throughout).
+ * FILTER_OFF scores every set exactly.  FILTER_ON changes nothing: the bound is
+ * the default (the value stays taken for callers that pass it). */
 #define EPISDET_FLAG_FILTER_ON 0x20u
 #define EPISDET_FLAG_FILTER_OFF 0x40u
 /* episdet_search_perm with order 2 on the tensor engine counts, per label,

@@ -259,7 +259,6 @@ struct LocalTopK {
         if (tid == 0) {
             *count = slot_count;
             *thr = (slot_count >= k) ? slot[k - 1] : cand_worst();
-            if (gkey && slot_count >= k) atomicMin(gkey, slot[k - 1].key);
         }
         bar();
     }

@@ -388,9 +388,9 @@ static int rate(int sms, int total, unsigned long long* d_cyc) {
     CK(cudaEventDestroy(e1));
     const double n = (double)groups * CPER;
     printf("{\"form\": \"pair\", \"n\": %d, \"mma_per_commit\": %d, \"issue\": \"%s\", \"ns_per_mma\": %.1f, "
-           "\"clk_per_mma\": %.1f, \"tmacs_per_s\": %.1f, \"err\": %d}\n",
+           "\"clk_per_mma\": %.1f, \"tmacs_per_s\": %.1f, \"sm_mhz\": %.0f, \"err\": %d}\n",
            N, COMMIT ? CPER : 0, ELECT ? "elected" : "one lane", best * 1e6 / n, cyc / n,
-           n * (sms / 2) * 256.0 * N * 64.0 / (best * 1e-3) / 1e12, err);
+           n * (sms / 2) * 256.0 * N * 64.0 / (best * 1e-3) / 1e12, cyc / (best * 1e3), err);  // the clock it ran at
     return err ? 1 : 0;
 }
 

@@ -60,15 +60,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
 }
 
-// 2-D TMA tile load global -> shared, completion counted on `bar` (bytes).
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::
-            "r"(smem_u32(dst)),
-        "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
-        : "memory");
-}
-
 // Bulk prefetch of [addr, addr + bytes) into L2 (16-byte aligned, bytes a multiple of 16).
 __device__ __forceinline__ void prefetch_l2(const void* addr, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(addr), "r"(bytes) : "memory");
@@ -107,17 +98,6 @@ __device__ __forceinline__ void tc_fence_before() {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// D[tmem] (+)= A[smem] * B[smem]^T, unsigned 8-bit inputs, s32 accumulate.
-__device__ __forceinline__ void mma_u8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                       uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 
 // Arrives once on `bar` when every tcgen05.mma issued so far by this thread completes.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -171,11 +151,6 @@ __device__ __forceinline__ bool elect_one() {
 // 128 bytes, 8-row groups 1024 bytes apart (SBO), descriptor version 1.
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
     return (uint64_t)((saddr & 0x3FFFF) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-
-// Instruction descriptor, kind::i8: D s32, A/B unsigned 8-bit, both K-major, M = m, N = n.
-__host__ __device__ constexpr uint32_t idesc_u8(uint32_t n, uint32_t m = 128) {
-    return (2u << 4) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
 // ---- CTA pairs (cluster of 2, cta_group::2) -------------------------------

@@ -25,7 +25,7 @@ ENGINE_AUTO, ENGINE_TENSOR, ENGINE_SIMT = 0, 1, 2
 FLAG_PROGRESS, FLAG_NO_VALIDATE, FLAG_TIMING = 0x1, 0x2, 0x4
 FLAG_AUTOTUNE = 0x8  # measure the triplet instance per shape and cache the choice
 FLAG_INJECT_STALL = 0x10  # testing aid: every tensor launch waits on a word nothing sets and times out
-FLAG_FILTER_ON, FLAG_FILTER_OFF = 0x20, 0x40  # bound scores before exact scoring (the default) / score every set exactly
+FLAG_FILTER_ON, FLAG_FILTER_OFF = 0x20, 0x40  # the default (scores bounded first) / score every set exactly
 FLAG_PERM_SPLIT = 0x80  # permutation search: a plain two-class search per label instead of label mode
 
 STATUS = {
