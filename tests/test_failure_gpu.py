@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("order,M,nc,nn", [(3, 40, 3000, 2500), (3, 12, 33000, 34000), (2, 300, 5000, 4000)],
-                         ids=["triplets", "triplets-staged", "pairs"])
+                         ids=["triplets", "triplets-large-classes", "pairs"])
 def test_stalled_launches_time_out_and_the_device_recovers(episdet, oracle, order, M, nc, nn):
     cases, controls = episdet.generate(0xFA11 + M, M, nc, nn)
     with pytest.raises(episdet.EpisdetError) as e:

@@ -28,9 +28,9 @@ def test_y_blocks_give_the_whole_table_answer(episdet, oracle, data1000, score, 
     k = 512
     o = oracle.search(cases, controls, 3000, 2800, order=3, score=score, top_k=k, first_begin=fb, first_end=fe)
     # 128 (the smallest block), 384 (a block edge inside a band of tiles) and a
-    # block of the whole range (the whole table); K2 also with the scoring filter.
+    # block of the whole range (the whole table); K2 also without the score bound.
     for blk in (128, 384, 1000):
-        for flags in ((0, episdet.FLAG_FILTER_ON) if score == "k2" else (0,)):
+        for flags in ((0, episdet.FLAG_FILTER_OFF) if score == "k2" else (0,)):
             r = episdet.search(cases, controls, 3000, 2800, order=3, score=score, top_k=k, engine="tensor",
                                first_begin=fb, first_end=fe, flags=flags, pair_block_snps=blk)
             assert_same(r, o, k)

@@ -42,9 +42,8 @@ def test_bench_workload_slabs(episdet, oracle, cfg2, slab):
     k = 1024
     o = oracle.search(cases, controls, CFG2["nc"], CFG2["nn"], order=3, score="k2", top_k=k, first_begin=fb,
                       first_end=fe)
-    # Both K2 triplet kernels: exact scoring, and the scoring filter (which a
-    # full search of this size runs).
-    for flags in (episdet.FLAG_FILTER_OFF, episdet.FLAG_FILTER_ON):
+    # Every set scored exactly, and the score bound (the default).
+    for flags in (episdet.FLAG_FILTER_OFF, 0):
         r = episdet.search(cases, controls, CFG2["nc"], CFG2["nn"], order=3, score="k2", top_k=k, engine="tensor",
                            first_begin=fb, first_end=fe, flags=flags)
         assert_same(r, o, k)
@@ -71,7 +70,7 @@ def test_tile_list_and_band_edges(episdet, oracle, score):
     cases, controls = episdet.generate(0x5CA1E, M, nc, nn)
     k = 1024
     o = oracle.search(cases, controls, nc, nn, order=3, score=score, top_k=k, first_begin=250, first_end=260)
-    for flags in ((episdet.FLAG_FILTER_OFF, episdet.FLAG_FILTER_ON) if score == "k2" else (0,)):
+    for flags in (episdet.FLAG_FILTER_OFF, 0):
         r = episdet.search(cases, controls, nc, nn, order=3, score=score, top_k=k, engine="tensor",
                            first_begin=250, first_end=260, flags=flags)
         assert_same(r, o, k)
