@@ -81,6 +81,26 @@ def test_counts_past_16_bits(episdet, oracle, order, M, slab):
           flags=(0, episdet.FLAG_FILTER_OFF))
 
 
+@pytest.mark.parametrize("order,M,slab", [(3, 30, (0, 0)), (2, 40, (0, 0)), (2, 1500, (700, 702))])
+def test_counts_past_16_bits_mi(episdet, oracle, order, M, slab):
+    check(episdet, oracle, order, M, 170000, 150000, "mi", 64, maf=(0.3, 0.36), slab=slab,
+          flags=(0, episdet.FLAG_FILTER_OFF))
+
+
+@pytest.mark.parametrize("score", ["k2", "mi"])
+@pytest.mark.parametrize("nc", [20000, 80000])
+def test_permutations_past_16_bits(episdet, oracle, score, nc):
+    """Pair totals of 150,000 samples (32-bit counts, one class); 80,000 cases are
+    counted in 32 bits too, 20,000 in 16."""
+    n, M, k = 150000, 40, 50
+    planes = episdet.generate_cohort(31, M, n, maf=(0.3, 0.5))
+    labels = episdet.generate_labels(32, n, nc, 2)
+    got = episdet.search_perm(planes, n, labels, order=2, score=score, top_k=k)
+    for lab, r in zip(labels, got):
+        a, b, na, nb = oracle.split_by_label(planes, n, lab)
+        assert_same(r, oracle.search(a, b, na, nb, order=2, score=score, top_k=k), k)
+
+
 @pytest.mark.parametrize("score", ["k2", "mi"])
 def test_more_ties_than_the_merge_holds(episdet, oracle, score):
     """Every SNP the same: all scores equal, the smallest sets win."""

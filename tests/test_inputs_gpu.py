@@ -72,6 +72,25 @@ def test_cohort_padding_bits_are_not_counted(episdet, oracle, score):
             assert_same(r, o, k)
 
 
+@pytest.mark.parametrize("order,engine", [(2, "tensor"), (3, "tensor"), (3, "simt")])
+def test_device_planes_still_being_written_on_the_callers_stream(episdet, oracle, order, engine):
+    import torch
+
+    M, nc, nn, k = 70, 1500, 1300, 32
+    planes = episdet.generate(93, M, nc, nn)
+    new = [torch.from_numpy(p.view("int32")).cuda() for p in planes]
+    late = [torch.zeros_like(p) for p in new]
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(400_000_000)
+        for p, q in zip(late, new):
+            p.copy_(q)
+    assert not stream.query()
+    r = episdet.search(*late, nc, nn, order=order, top_k=k, engine=engine, stream=stream.cuda_stream)
+    assert_same(r, oracle.search(*planes, nc, nn, order=order, score="k2", top_k=k), k)
+
+
 def test_device_labels_still_being_written_on_the_callers_stream(episdet, oracle):
     """The labels (all zero until then) arrive on the caller's stream behind a
     wait of some tenths of a second, and are not what the buffer held before."""
