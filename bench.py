@@ -43,6 +43,14 @@ SEED = 0xE917
 PUBLISHED = 25.0  # the reference's published "> 25 x 10^12" on a GeForce RTX 2070 SUPER (README.md:54-61)
 METRIC = "3-way K2 tera (triplets×samples)/s at 4096 SNP×262144; batched vs plain"
 UNIT = "1e12 triplets*samples/s"
+# Rate of the counting kernel's instruction (tcgen05.mma.cta_group::2.kind::mxf4,
+# M = 256, N = 224: 112 clocks, 32768 MACs a clock and CTA pair) on 74 CTA pairs,
+# measured by episdet-peak-f4 over 0.6 s: 4473 TMAC/s, with nvidia-smi at 1965 MHz
+# and the SM's cycle counter at 1845.
+MXF4_PEAK_TFLOPS = 2 * 4473.0
+# DRAM bytes (read and written) per executed MAC of a steady triplet launch of the
+# workload below, from a one-pass capture: 14.35 GB over 1.78e13 MACs.
+DRAM_BYTES_PER_MAC = 8.05e-4
 WORKLOAD = ("exhaustive 3-way K2 search, 4096 SNPs x 262144 samples (131072 cases + 131072 controls), "
             "HWE genotypes MAF~U[0.05,0.5], planted triplet {137,2048,3901}")
 
@@ -359,22 +367,13 @@ def ours(args):
         return
     # Roofline of the dominant kernel (the triplet counting launches), this rank:
     # the e2m1 MACs it issues (2 ops each) per second of its launches, against
-    # the measured rate of its instruction at the shape it issues
-    # (tcgen05.mma.cta_group::2.kind::mxf4, N = 224, at the maximum SM clock;
-    # profiles/tcgen05_mma_peak.md), and beside it the N = 256 rate and the
-    # measured bf16 x 4 figure.
+    # the measured rate of its instruction at the shape it issues, and beside it
+    # the measured bf16 x 4 figure.
     peaks = {}
     pp = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(pp):
         peaks = json.load(open(pp))
     bf16 = peaks.get("bf16_tflops_sustained") or 1400.0
-    inst = {}
-    pk = os.path.join(ROOT, "profiles", "tcgen05_mma_peak.md")
-    if os.path.exists(pk):
-        for line in open(pk):
-            for key in ("mxf4_pair_n224_peak_tflops", "mxf4_pair_n256_peak_tflops"):
-                if line.startswith(key + ":"):
-                    inst[key] = float(line.split(":")[1].split()[0])
     kern_ms = sum(r.count_kernel_ms for r, _ in res) / args.steps
     launches = sum(r.count_kernel_launches for r, _ in res) / args.steps
     slab_sets = r0.sets_evaluated
@@ -382,14 +381,11 @@ def ours(args):
     exe_ops = 2.0 * r0.executed_macs
     algorithmic = alg_ops / (kern_ms * 1e-3) / 1e12
     executed = exe_ops / (kern_ms * 1e-3) / 1e12
-    peak = inst.get("mxf4_pair_n224_peak_tflops")
-    p256 = inst.get("mxf4_pair_n256_peak_tflops")
-    roof = {"bound": "tensor", "achieved": executed, "peak": peak, "unit": "TFLOP/s",
-            "frac": (executed / peak) if peak else None, "traffic": None,
+    roof = {"bound": "tensor", "achieved": executed, "peak": MXF4_PEAK_TFLOPS, "unit": "TFLOP/s",
+            "frac": executed / MXF4_PEAK_TFLOPS,
+            "traffic": DRAM_BYTES_PER_MAC * r0.executed_macs / max(launches, 1),
             "kernel": "episdet::tc::count_kernel (triplets)",
-            "peak_source": "measured: kind::mxf4 CTA-pair MMA, M=256 N=224, at 1965 MHz (profiles/tcgen05_mma_peak.md)",
-            "frac_of_n256_instruction_peak": (executed / p256) if p256 else None,
-            "n256_instruction_peak_tflops": p256,
+            "peak_source": "measured: kind::mxf4 CTA-pair MMA, M=256 N=224, nvidia-smi at 1965 MHz (episdet-peak-f4)",
             "frac_of_4x_bf16_sustained": executed / (4.0 * bf16),
             "algorithmic_tflops": algorithmic,
             "kernel_ms_per_step": kern_ms, "launches_per_step": launches,
@@ -397,11 +393,6 @@ def ours(args):
             "note": "achieved = e2m1 MACs the kernel issues x 2 / its launch time; the engine regroups samples by "
                     "the first SNP's genotype (exact), so it issues 4.2x fewer MACs than the algorithmic 8 AND "
                     "cells x N per triplet counted in algorithmic_tflops"}
-    prof = os.path.join(ROOT, "profiles", "count_kernel_triplets.md")
-    if os.path.exists(prof):
-        for line in open(prof):
-            if line.startswith("traffic_bytes_per_launch_scaled:"):
-                roof["traffic"] = float(line.split(":")[1].split()[0])
     out = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "strong",
