@@ -18,18 +18,19 @@
 //   warps 6-13   scoring: read the tile's counts back, one set per lane, bound
 //                every score, score the survivors.
 //
-// Why this split (measured on a B200, SM at its 1965 MHz maximum): the MMA
-// itself takes N / 2 clocks (56 for N = 112, 112 for N = 224) whatever the
-// number of MMAs per commit, 4430 TMAC/s on the chip, so the tensor pipe wants
-// MMAs back to back and operands at 64 bytes per clock and SM.  A tile of N =
-// 112 needs 103 (4 KB of A and 1.75 KB of B per 56 clocks), one of N = 224
-// needs 67.  With all four segments of a triplet tile in TMEM at once N cannot
+// Why this split (measured on a B200): the MMA itself takes N / 2 clocks (56 for
+// N = 112, 112 for N = 224) whatever the number of MMAs per commit, 4470 TMAC/s
+// on the chip (nvidia-smi at 1965 MHz, the SM's cycle counter at 1845), so the
+// tensor pipe wants MMAs back to back and operands at 64 bytes per clock and SM.
+// A tile of N = 112 needs 103 (4 KB of A and 1.75 KB of B per 56 clocks), one of
+// N = 224 needs 67.  With all four segments of a triplet tile in TMEM at once N cannot
 // pass 112, and the scoring of a tile holds its accumulators; moving finished
 // segments out costs 57 KB of L2 traffic each (against 1 to 4 MB of operands)
 // and frees both N and the issuer.  One eighth of the 4096 x 262144 K2 search: 531
-// ms with four segments in TMEM and exact scoring beside them, 250 ms so; one
-// sixteenth of the 8192 x 65536 MI search 750 -> 297 ms; 1536 SNPs x 40000 samples
-// K2 132 -> 39 ms; all pairs of 16384 SNPs x 32768 samples MI 12.1 -> 5.5 ms.
+// ms with four segments in TMEM and exact scoring beside them, 259 ms so; one
+// sixteenth of the 8192 x 65536 MI search 750 -> 320 ms; 1536 SNPs x 40000 samples
+// K2 132 -> 40 ms; all pairs of 16384 SNPs x 32768 samples MI 12.1 -> 6.1 ms
+// (repeated for seconds, under the power cap).
 #pragma once
 #include <cuda.h>
 
