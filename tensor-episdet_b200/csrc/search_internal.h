@@ -107,6 +107,10 @@ struct Workspace {
     std::vector<double> launch_ms, launch_macs;  // EPISDET_FLAG_TIMING: per counting launch of the last call
     int tab_score = -1, tab_size = 0, tab_nc = -1, tab_nn = -1;
     int stage_override = -1;  // triplet tiles: -1 by the panel-size rule, 0 narrow, 1 wide
+    // The first SNPs of a launch that memory last allowed, for regrouped rows of
+    // limit_bytes a first SNP; asked again after limit_uses searches.
+    size_t limit_bytes = 0;
+    int limit = 0, limit_uses = 0;
     int pairs[16] = {};       // resident CTA pairs of each counting-kernel instance (0: not asked yet)
     float inv32 = 0.0f, hy32 = 0.0f;
     double inv64 = 0.0, hy64 = 0.0;
@@ -121,6 +125,7 @@ struct Workspace {
                          &bin_geno, &bin_idx, &bin_pack, &bin_out[0], &bin_out[1]};
         for (DevBuf* b : all) b->release();
         results.release();
+        limit_uses = 0;
         tab_score = tab_nc = tab_nn = -1;
     }
 };

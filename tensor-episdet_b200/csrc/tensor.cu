@@ -998,13 +998,25 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
             return more;
         };
         auto table_bytes = [&] { return row_bytes * (blk_tiles < all_tiles ? (size_t)blk_tiles * kTileA : (size_t)M); };
+        auto keep_limit = [&](int top) {
+            w->limit_bytes = member_bytes;
+            w->limit = gmax;
+            w->limit_uses = gmax < top ? 64 : 0;
+        };
         // Chooses gmax and, unless asked for, the pair table's blocks.  (Free
         // memory is asked for only when something has to grow: on some hosts the
         // driver takes 9 ms to answer, more than a small search.)
         auto plan = [&]() -> episdet_status {
+            const int top = gmax;
             const bool asked = blk_tiles < all_tiles;
             const bool held_all = w->ptab.cap >= table_bytes() && (!asked || w->ptabx.cap >= xrows_bytes);
             if (held_all && growth(gmax) == 0) return EPISDET_OK;
+            // A launch size that memory limited lately is kept for searches with the same rows.
+            if (held_all && w->limit_bytes == member_bytes && w->limit_uses > 0 && growth(std::min(gmax, w->limit)) == 0) {
+                --w->limit_uses;
+                gmax = std::min(gmax, w->limit);
+                return EPISDET_OK;
+            }
             size_t fr = 0, tot = 0;
             CUDA_TRY(cudaMemGetInfo(&fr, &tot));
             // Left for the tile lists, slots, merge buffers and the driver.
@@ -1014,15 +1026,25 @@ episdet_status run_tensor(Workspace* w, DevData& D, const ScoreTables& T, const 
             size_t held = held_all ? 0 : w->ptab.cap + w->ptabx.cap;
             const size_t least = reserve + table + growth(kXGroup);
             if (fr + held >= least) {
-                // Larger launches take a small part of what is left, so that they
-                // narrow nothing for the other lanes of a batch or other processes.
-                const size_t spare = (fr + held - least) / 16;
-                while (gmax > kXGroup && growth(gmax) > growth(kXGroup) + spare) gmax = std::max(kXGroup, gmax * 3 / 4);
+                // Larger launches hold a small part of what is left beside the smallest,
+                // so that they narrow nothing for the other lanes of a batch or other
+                // processes; what they hold already is part of what is left.
+                size_t spare = fr + held - least;
+                for (const Need& d : needs(kXGroup)) spare += d.buf->cap > d.bytes ? d.buf->cap - d.bytes : 0;
+                auto total = [&](int g) {
+                    size_t b = 0;
+                    for (const Need& d : needs(g)) b += d.bytes;
+                    return b;
+                };
+                while (gmax > kXGroup && growth(gmax) > 0 && total(gmax) > total(kXGroup) + spare / 16)
+                    gmax = std::max(kXGroup, gmax * 3 / 4);
+                keep_limit(top);
                 return EPISDET_OK;
             }
             // Little memory left: the smallest launches, and what earlier searches'
             // larger ones hold goes back.
             gmax = kXGroup;
+            keep_limit(top);
             for (const Need& d : needs(gmax))
                 if (d.buf->cap > d.bytes) d.buf->release();
             if (asked || held_all) return EPISDET_OK;

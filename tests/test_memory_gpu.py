@@ -58,6 +58,33 @@ def test_little_free_memory(episdet, oracle, fresh):
     assert r.count_kernel_launches == 2  # 4 first SNPs a launch, one pass over them
 
 
+def test_limited_launches_stay_as_they_are(episdet, oracle, fresh):
+    """With 12 GB free the launches take a few first SNPs more than the smallest;
+    repeated searches take the same and no more memory, and a later one with room
+    takes all."""
+    import torch
+
+    M, nc, nn, k = 1500, 20000, 20000, 64
+    data = episdet.generate(0x8E, M, nc, nn)
+    kw = dict(order=3, top_k=k, engine="tensor", first_begin=0, first_end=32)
+    episdet.search(*data, nc, nn, order=2, top_k=k)
+    episdet.release_workspace(0)
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (12 << 30), dtype=torch.uint8, device="cuda")
+    try:
+        seen = []
+        for _ in range(3):
+            r = episdet.search(*data, nc, nn, **kw)
+            seen.append((r.count_kernel_launches, torch.cuda.mem_get_info()[0]))
+    finally:
+        del hold
+    assert 1 < seen[0][0] < 8 and seen == seen[:1] * 3
+    torch.cuda.empty_cache()
+    for _ in range(70):
+        r = episdet.search(*data, nc, nn, **dict(kw, first_end=8))
+    assert r.count_kernel_launches == 1
+    assert_same(r, oracle.search(*data, nc, nn, order=3, score="k2", top_k=k, first_begin=0, first_end=8), k)
+
+
 def test_room_held_by_larger_launches_is_given_back(episdet, oracle, fresh):
     """After a search whose launches hold 4 GB, one whose pair table (2.9 GB) does
     not fit beside them: they go, not the whole table."""
